@@ -383,10 +383,7 @@ __global__ void k_fixed_to_grid_cp(const long long* q, int NP, int64_t cells, co
   const int nc = cells - cell0 < 32 ? (int)(cells - cell0) : 32;
   for (int e = threadIdx.x; e < nc * NP; e += blockDim.x) {
     const int c = e / NP, p = e - c * NP;
-    const long long v = q[(cell0 + c) * NP + p];
-    const long long hi = (v + (1ll << 31)) >> 32;
-    const int lo = (int)(v - hi * 4294967296ll);
-    tile[c][p] = __fmaf_rn((float)(int)hi, 4294967296.f, (float)lo) * inv;
+    tile[c][p] = fx_to_float(q[(cell0 + c) * NP + p]) * inv;
   }
   __syncthreads();
   const int nch = NP / 2;
@@ -426,45 +423,50 @@ __device__ __forceinline__ void es_axis(float k, int M, float* w, int* idx) {
   }
 }
 
-// ------------------------------------------------- tile-sorted (2D) ---
+// ------------------------------------------------------ tile sorts ---
 //
-// 2D grids are spread tile by tile.  Samples are counting-sorted by the 12 x 12 tile that
-// holds their first tap; a work item is a chunk of up to kChunk samples of one tile and a
-// group of P accumulator parts (a part is the real or the imaginary plane of a channel).
-// A CTA sums its item into a shared-memory window of (12 + w - 1)^2 cells x P parts, then
-// adds every nonzero window cell to the grid with one global 64-bit atomic, the lanes of a
-// warp on consecutive cells of a window row (one coalesced flush per window row and part).
-//
-// Lanes own parts, not taps: a sample's value for each part is formed once, and its 64
-// terms are that value times the separable tap weights, each added at a window offset
-// fixed at compile time.  The terms are the fixed-point terms of the global kernels
-// (|term| < 2^40) and enter the window as their two fx_split limbs, round(a) and the
-// 21-bit remainder: 32-bit shared atomics run at ~5x the rate of 64-bit ones, and the
-// limb sums of at most kChunk terms cannot overflow (|low sums| <= 2^30, |high sums| <
-// 2^30).  The flush rebuilds each window cell's exact 64-bit sum from its limbs, so every
-// grid cell is the exact integer sum of its rounded terms, whatever order the samples and
-// items land in: the grids are reproducible run to run.
-constexpr int kTile = 12;
+// Samples counting-sorted by the tile (kTile or kSpTile cells a side, 2D and 3D) that holds
+// their first tap; a work item is a chunk of samples of one tile.  The samples are counted in
+// at most kSegs segments of consecutive ones, and a chunk takes whole segments of its tile, as
+// many as fit; a segment of a tile with more samples than a chunk takes is put in order first
+// (k_tile_order) and cut.  So which samples a chunk holds does not depend on the order in which
+// the atomics land; their order inside it does.  (The interpolation, where a sample's result
+// does not depend on its chunk, takes one segment and no order.)
+constexpr int kSegs = 64;
+constexpr int kSegMin = 8192;               // samples per segment, at least
+constexpr int kTile = 12;                   // 2D interpolation windows
 constexpr int kWin = kTile + kEsWidth - 1;  // 19
-constexpr int kWinCells = kWin * kWin;      // 361: odd, so the part stride is bank-conflict free
-constexpr int kChunk = 1024;                // samples per work item
+constexpr int kWinCells = kWin * kWin;      // 361
+constexpr int kChunk = 1024;                // samples per work item of the interpolation kernels
 constexpr int kTiledThreads = 512;
-static_assert(kChunk * (1ll << (kFxLoBits - 1)) < (1ll << 31), "low limb sums must fit in 31 bits");
-static_assert(kChunk * (1ll << (kFxTermBits - kFxLoBits)) < (1ll << 31), "high limb sums must fit in 31 bits");
 
-template <int P>
-constexpr int tiled_smem_bytes() { return 2 * P * kWinCells * (int)sizeof(int); }
+// Counts the samples of a warp per tile: one atomic per run of equal tiles (neighbours along a
+// trajectory share a tile).  Returns the sample's place among its tile's, given the counter's
+// value before.
+__device__ __forceinline__ int tile_count(int* counter, int t, bool act) {
+  const int lane = threadIdx.x & 31;
+  const unsigned grp = __match_any_sync(0xffffffffu, act ? t : -1);
+  const int lead = __ffs(grp) - 1;
+  int base = 0;
+  if (act && lane == lead) base = atomicAdd(&counter[t], __popc(grp));
+  base = __shfl_sync(0xffffffffu, base, lead);
+  return base + __popc(grp & ((1u << lane) - 1u));
+}
 
 // home tile of every kept sample: the tile holding its first tap (l0 of es_lane_weight)
-__global__ void k_tile_home(SampleSet S, int M0, int M1, int ntx, int* tile_of, int* counts) {
+__global__ void k_tile_home(SampleSet S, int M0, int M1, int M2, int tile, int64_t seg, int ntiles, int* tile_of,
+                            int* counts) {
   const int hw = kEsWidth / 2;
-  const int M[2] = {M0, M1};
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < S.n; n += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t li = sample_lin(S, n);
-    int l0[2];
-    for (int dd = 0; dd < 2; ++dd) {
+  const int M[3] = {M0, M1, M2};
+  const int ntx = (M0 + tile - 1) / tile, nty = (M1 + tile - 1) / tile;
+  for (int64_t n0 = blockIdx.x * (int64_t)blockDim.x; n0 < S.n; n0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t n = n0 + threadIdx.x;
+    const bool act = n < S.n;
+    const int64_t li = act ? sample_lin(S, n) : 0;
+    int l0[3] = {0, 0, 0};
+    for (int dd = 0; dd < S.d; ++dd) {
       const float m = (float)M[dd];
-      const float kd = S.trj[dd + 2 * li];
+      const float kd = act ? S.trj[dd + (int64_t)S.d * li] : 0.f;
       const float uh = __fmul_rn(kd, m);  // the arithmetic of es_lane_weight, operation for operation
       const float ul = fmaf(kd, m, -uh);
       const float f = floorf(uh);
@@ -472,57 +474,140 @@ __global__ void k_tile_home(SampleSet S, int M0, int M1, int ntx, int* tile_of, 
       int l = ((int)f - hw + (r > 0.f ? 1 : 0)) % M[dd];
       l0[dd] = l < 0 ? l + M[dd] : l;
     }
-    const int t = l0[0] / kTile + ntx * (l0[1] / kTile);
-    tile_of[n] = t;
-    atomicAdd(&counts[t], 1);
+    const int t = l0[0] / tile + ntx * (l0[1] / tile + nty * (l0[2] / tile));
+    if (act) tile_of[n] = t;
+    tile_count(counts + (n0 / seg) * ntiles, t, act);  // seg is a multiple of the block
+  }
+}
+
+// Walks tile t's segments (counts[segment][tile]): each(segment, samples), and chunk(first,
+// count) per work item, positions counted from `first`.
+template <class Each, class Chunk>
+__device__ __forceinline__ void tile_chunks(const int* counts, int nseg, int ntiles, int t, int first, int most, Each each,
+                                            Chunk chunk) {
+  int cur = 0;
+  for (int g = 0; g < nseg; ++g) {
+    const int c = counts[(int64_t)g * ntiles + t];
+    each(g, c);
+    if (c == 0) continue;
+    if (cur != 0 && cur + c > most) {
+      chunk(first, cur);
+      first += cur;
+      cur = 0;
+    }
+    cur += c;
+    while (cur > most) {
+      chunk(first, most);
+      first += most;
+      cur -= most;
+    }
+  }
+  if (cur != 0) chunk(first, cur);
+}
+
+// per tile: samples and chunks over its segments
+__global__ void k_tile_chunks(const int* counts, int nseg, int ntiles, int most, int* total, int* nch) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
+    int sum = 0, n = 0;
+    tile_chunks(counts, nseg, ntiles, t, 0, most, [&](int, int c) { sum += c; }, [&](int, int) { ++n; });
+    total[t] = sum;
+    nch[t] = n;
   }
 }
 
 // one block: offsets of the tiles' sample lists and of their chunks, and the chunk count
-__global__ void __launch_bounds__(1024) k_tile_scan(const int* counts, int ntiles, int* offset, int* choff,
+__global__ void __launch_bounds__(1024) k_tile_scan(const int* total, const int* nch, int ntiles, int* offset, int* choff,
                                                     int* nitems) {
-  __shared__ int s_n[1024], s_c[1024];
-  const int per = (ntiles + blockDim.x - 1) / blockDim.x;
-  const int t0 = threadIdx.x * per, t1 = min(ntiles, t0 + per);
-  int sn = 0, sc = 0;
-  for (int t = t0; t < t1; ++t) {
-    sn += counts[t];
-    sc += (counts[t] + kChunk - 1) / kChunk;
-  }
-  s_n[threadIdx.x] = sn;
-  s_c[threadIdx.x] = sc;
-  __syncthreads();
-  for (int o = 1; o < (int)blockDim.x; o <<= 1) {  // inclusive Hillis-Steele scan
-    const int an = threadIdx.x >= (unsigned)o ? s_n[threadIdx.x - o] : 0;
-    const int ac = threadIdx.x >= (unsigned)o ? s_c[threadIdx.x - o] : 0;
+  __shared__ int s_n[32], s_c[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int bn = 0, bc = 0;  // totals of the tiles before this round's
+  for (int t0 = 0; t0 < ntiles; t0 += 1024) {
+    const int t = t0 + threadIdx.x;
+    const int vn = t < ntiles ? total[t] : 0, vc = t < ntiles ? nch[t] : 0;
+    int xn = vn, xc = vc;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int yn = __shfl_up_sync(0xffffffffu, xn, o), yc = __shfl_up_sync(0xffffffffu, xc, o);
+      if (lane >= o) {
+        xn += yn;
+        xc += yc;
+      }
+    }
+    if (lane == 31) {
+      s_n[warp] = xn;
+      s_c[warp] = xc;
+    }
     __syncthreads();
-    s_n[threadIdx.x] += an;
-    s_c[threadIdx.x] += ac;
+    int wn = 0, wc = 0, an = 0, ac = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) {
+        wn += s_n[w];
+        wc += s_c[w];
+      }
+      an += s_n[w];
+      ac += s_c[w];
+    }
+    if (t < ntiles) {
+      offset[t] = bn + wn + xn - vn;
+      choff[t] = bc + wc + xc - vc;
+    }
+    bn += an;
+    bc += ac;
     __syncthreads();
   }
-  int on = s_n[threadIdx.x] - sn, oc = s_c[threadIdx.x] - sc;
-  for (int t = t0; t < t1; ++t) {
-    offset[t] = on;
-    choff[t] = oc;
-    on += counts[t];
-    oc += (counts[t] + kChunk - 1) / kChunk;
-  }
-  if (threadIdx.x == blockDim.x - 1) *nitems = s_c[threadIdx.x];
+  if (threadIdx.x == 0) *nitems = bc;
 }
 
-__global__ void k_tile_scatter(int64_t n, const int* tile_of, const int* offset, int* cursor, int* order) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int t = tile_of[i];
-    order[offset[t] + atomicAdd(&cursor[t], 1)] = (int)i;
-  }
-}
-
-__global__ void k_tile_items(const int* counts, const int* offset, const int* choff, int ntiles, int4* items) {
+// per tile: its segments' places in the sorted order (written over counts), its work items
+// (tile, first sorted position, count, -) and the segments with more samples than a chunk takes
+__global__ void k_tile_items(int* counts, int nseg, int ntiles, int most, const int* offset, const int* choff, int4* items,
+                             int2* big, int* nbig) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
-    const int c = counts[t];
-    for (int j = 0; j * kChunk < c; ++j)
-      items[choff[t] + j] = make_int4(t, offset[t] + j * kChunk, min(kChunk, c - j * kChunk), 0);
+    int pos = offset[t], ch = choff[t];
+    tile_chunks(counts, nseg, ntiles, t, pos, most,
+                [&](int g, int c) {
+                  counts[(int64_t)g * ntiles + t] = pos;
+                  if (c > most) big[atomicAdd(nbig, 1)] = make_int2(pos, c);
+                  pos += c;
+                },
+                [&](int first, int c) { items[ch++] = make_int4(t, first, c, 0); });
   }
+}
+
+// Puts the samples of the `big` segments in order (each one's place is the number of smaller
+// ones), a block each; tmp: room for all samples.
+__global__ void __launch_bounds__(1024) k_tile_order(const int2* big, const int* nbig, int* order, int* tmp) {
+  for (int b = blockIdx.x; b < *nbig; b += gridDim.x) {
+    const int2 s = big[b];
+    for (int i = threadIdx.x; i < s.y; i += blockDim.x) tmp[s.x + i] = order[s.x + i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < s.y; i += blockDim.x) {
+      const int v = tmp[s.x + i];
+      int r = 0;
+      for (int j = 0; j < s.y; ++j) r += tmp[s.x + j] < v;
+      order[s.x + r] = v;
+    }
+  }
+}
+
+__global__ void k_tile_scatter(int64_t n, int64_t seg, int ntiles, const int* tile_of, int* cursor, int* order) {
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = i0 + threadIdx.x;
+    const bool act = i < n;
+    const int place = tile_count(cursor + (i0 / seg) * ntiles, act ? tile_of[i] : 0, act);
+    if (act) order[place] = (int)i;
+  }
+}
+
+// Density compensation of kept sample n at linear index li (src/BackProjection.jl:169-181).
+__device__ __forceinline__ float sample_dcf(const SampleSet& S, int64_t n, int64_t li, int kind, const float* dcf) {
+  if (kind == MRSR_DCF_ARRAY) return dcf[n];
+  if (kind != MRSR_DCF_RADIAL_3D && kind != MRSR_DCF_RADIAL_2D) return 1.f;
+  float s2 = 0.f;
+  for (int dd = 0; dd < S.d; ++dd) {
+    const float k = S.trj[dd + (int64_t)S.d * li];
+    s2 = __fadd_rn(s2, __fmul_rn(k, k));
+  }
+  return kind == MRSR_DCF_RADIAL_3D ? s2 : sqrtf(s2);
 }
 
 // Per-sample tap record of the tile-sorted kernels, in sorted order: the separable weights
@@ -544,13 +629,7 @@ __global__ void k_tile_prep(SampleSet S, int M0, int M1, const int* order, int d
     int ix[kEsWidth], iy[kEsWidth];
     es_axis(k0, M0, r.wx, ix);
     es_axis(k1, M1, r.wy, iy);
-    float w = 1.f;
-    if (dcf_kind == MRSR_DCF_RADIAL_3D || dcf_kind == MRSR_DCF_RADIAL_2D) {
-      const float s2 = __fadd_rn(__fmul_rn(k0, k0), __fmul_rn(k1, k1));
-      w = dcf_kind == MRSR_DCF_RADIAL_3D ? s2 : sqrtf(s2);
-    } else if (dcf_kind == MRSR_DCF_ARRAY) {
-      w = dcf[n];
-    }
+    const float w = sample_dcf(S, n, li, dcf_kind, dcf);
 #pragma unroll
     for (int j = 0; j < kEsWidth; ++j) r.wy[j] *= w;
     r.li = (int)li;
@@ -562,6 +641,7 @@ __global__ void k_tile_prep(SampleSet S, int M0, int M1, const int* order, int d
 }
 
 int TileSort::prep(const SampleSet& S, int dcf_kind, const float* dcf, cudaStream_t st) {
+  if (S.d == 3) return prep3(S, dcf_kind, dcf, st);
   MRSR_REQUIRE(S.ns_pf * S.nt < (1ll << 31), MRSR_ERR_UNSUPPORTED, "tile records: < 2^31 samples per set");
   MRSR_TRY(rec.alloc(sizeof(TapRec) * std::max<int64_t>(S.n, 1)));
   const unsigned gb = (unsigned)std::min<int64_t>(std::max<int64_t>(cdiv(S.n, 256), 1), 152 * 16);
@@ -570,99 +650,63 @@ int TileSort::prep(const SampleSet& S, int dcf_kind, const float* dcf, cudaStrea
   return MRSR_OK;
 }
 
-int TileSort::build(const SampleSet& S, int64_t M0, int64_t M1, cudaStream_t st) {
-  MRSR_REQUIRE(S.d == 2 && S.n < (1ll << 31) && M0 < (1ll << 24) && M1 < (1ll << 24), MRSR_ERR_UNSUPPORTED,
-               "tile-sorted spreading: 2D, < 2^31 samples, grid < 2^24 per dimension");
-  ntx = (int)cdiv(M0, kTile);
-  ntiles = ntx * (int)cdiv(M1, kTile);
-  m0 = (int)M0;
-  m1 = (int)M1;
-  const int64_t maxitems = ntiles + cdiv(S.n, kChunk);
-  MRSR_TRY(counts.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(offset.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(choff.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(cursor.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(tile_of.alloc(sizeof(int) * std::max<int64_t>(S.n, 1)));
-  MRSR_TRY(order.alloc(sizeof(int) * std::max<int64_t>(S.n, 1)));
-  MRSR_TRY(items.alloc(sizeof(int4) * maxitems));
-  MRSR_TRY(nitems.alloc(sizeof(int)));
-  MRSR_TRY(next.alloc(sizeof(int)));
-  MRSR_CHECK_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * ntiles, st));
-  MRSR_CHECK_CUDA(cudaMemsetAsync(cursor.p, 0, sizeof(int) * ntiles, st));
-  const unsigned gb = (unsigned)std::min<int64_t>(std::max<int64_t>(cdiv(S.n, 256), 1), 152 * 16);
-  k_tile_home<<<gb, 256, 0, st>>>(S, m0, m1, ntx, tile_of.as<int>(), counts.as<int>());
-  MRSR_LAUNCH_CHECK();
-  k_tile_scan<<<1, 1024, 0, st>>>(counts.as<int>(), ntiles, offset.as<int>(), choff.as<int>(), nitems.as<int>());
-  MRSR_LAUNCH_CHECK();
-  k_tile_scatter<<<gb, 256, 0, st>>>(S.n, tile_of.as<int>(), offset.as<int>(), cursor.as<int>(), order.as<int>());
-  MRSR_LAUNCH_CHECK();
-  const unsigned gt = (unsigned)std::max<int64_t>(cdiv(ntiles, 256), 1);
-  k_tile_items<<<gt, 256, 0, st>>>(counts.as<int>(), offset.as<int>(), choff.as<int>(), ntiles, items.as<int4>());
-  MRSR_LAUNCH_CHECK();
-  return MRSR_OK;
-}
-
-constexpr int kTile3 = 8;
-
-// 3D home tile (kTile3^3) of every kept sample's first tap
-__global__ void k_tile_home3(SampleSet S, int M0, int M1, int M2, int* tile_of, int* counts) {
-  const int hw = kEsWidth / 2;
-  const int M[3] = {M0, M1, M2};
-  const int ntx = (M0 + kTile3 - 1) / kTile3, nty = (M1 + kTile3 - 1) / kTile3;
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < S.n; n += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t li = sample_lin(S, n);
-    int l0[3];
-    for (int dd = 0; dd < 3; ++dd) {
-      const float m = (float)M[dd];
-      const float kd = S.trj[dd + 3 * li];
-      const float uh = __fmul_rn(kd, m);
-      const float ul = fmaf(kd, m, -uh);
-      const float f = floorf(uh);
-      const float r = __fadd_rn(__fsub_rn(uh, f), ul);
-      int l = ((int)f - hw + (r > 0.f ? 1 : 0)) % M[dd];
-      l0[dd] = l < 0 ? l + M[dd] : l;
-    }
-    const int t = l0[0] / kTile3 + ntx * (l0[1] / kTile3 + nty * (l0[2] / kTile3));
-    tile_of[n] = t;
-    atomicAdd(&counts[t], 1);
-  }
-}
-
-int TileSort::build3(const SampleSet& S, const int64_t* M, cudaStream_t st) {
-  MRSR_REQUIRE(S.d == 3 && S.n < (1ll << 31), MRSR_ERR_UNSUPPORTED, "sample order: 3D, < 2^31 samples");
-  const int64_t nt3 = cdiv(M[0], kTile3) * cdiv(M[1], kTile3) * cdiv(M[2], kTile3);
-  MRSR_REQUIRE(nt3 < (1ll << 31), MRSR_ERR_UNSUPPORTED, "sample order: too many tiles");
-  ntiles = (int)nt3;
-  MRSR_TRY(counts.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(offset.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(choff.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(cursor.alloc(sizeof(int) * ntiles));
-  MRSR_TRY(tile_of.alloc(sizeof(int) * std::max<int64_t>(S.n, 1)));
-  MRSR_TRY(order.alloc(sizeof(int) * std::max<int64_t>(S.n, 1)));
-  MRSR_TRY(nitems.alloc(sizeof(int)));
-  MRSR_CHECK_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * ntiles, st));
-  MRSR_CHECK_CUDA(cudaMemsetAsync(cursor.p, 0, sizeof(int) * ntiles, st));
-  const unsigned gb = (unsigned)std::min<int64_t>(std::max<int64_t>(cdiv(S.n, 256), 1), 152 * 16);
-  k_tile_home3<<<gb, 256, 0, st>>>(S, (int)M[0], (int)M[1], (int)M[2], tile_of.as<int>(), counts.as<int>());
-  MRSR_LAUNCH_CHECK();
-  k_tile_scan<<<1, 1024, 0, st>>>(counts.as<int>(), ntiles, offset.as<int>(), choff.as<int>(), nitems.as<int>());
-  MRSR_LAUNCH_CHECK();
-  k_tile_scatter<<<gb, 256, 0, st>>>(S.n, tile_of.as<int>(), offset.as<int>(), cursor.as<int>(), order.as<int>());
-  MRSR_LAUNCH_CHECK();
-  // work items of the 3D tile-sorted kernel: chunks of at most kChunk samples of one tile
+int TileSort::build(const SampleSet& S, const int64_t* M, int tile_, int most, bool stable, cudaStream_t st) {
+  MRSR_REQUIRE(S.n < (1ll << 31), MRSR_ERR_UNSUPPORTED, "tile sort: < 2^31 samples");
+  const int64_t nt = cdiv(M[0], tile_) * cdiv(M[1], tile_) * (S.d == 3 ? cdiv(M[2], tile_) : 1);
+  MRSR_REQUIRE(nt < (1ll << 31) && M[0] < (1ll << 24) && M[1] < (1ll << 24) && (S.d == 2 || M[2] < (1ll << 24)),
+               MRSR_ERR_UNSUPPORTED, "tile sort: too many tiles");
+  tile = tile_;
+  ntiles = (int)nt;
+  ntx = (int)cdiv(M[0], tile);
+  nty = (int)cdiv(M[1], tile);
   m0 = (int)M[0];
   m1 = (int)M[1];
-  m2 = (int)M[2];
-  ntx = (int)cdiv(M[0], kTile3);
-  nty = (int)cdiv(M[1], kTile3);
-  const int64_t maxitems = ntiles + cdiv(S.n, kChunk);
+  m2 = S.d == 3 ? (int)M[2] : 1;
+  const int64_t seg = cdiv(stable ? std::max<int64_t>(kSegMin, cdiv(S.n, kSegs)) : std::max<int64_t>(S.n, 1), 256) * 256;
+  const int nseg = (int)std::max<int64_t>(1, cdiv(S.n, seg));
+  // two neighbouring chunks of a tile hold more than `most` samples
+  const int64_t maxitems = ntiles + 2 * cdiv(S.n, most);
+  DevBuf big, nbig, tmp;
+  MRSR_TRY(big.alloc(sizeof(int2) * (size_t)(S.n / most + 1)));
+  MRSR_TRY(nbig.alloc(sizeof(int)));
+  if (stable) MRSR_TRY(tmp.alloc(sizeof(int) * std::max<int64_t>(S.n, 1)));
+  MRSR_CHECK_CUDA(cudaMemsetAsync(nbig.p, 0, sizeof(int), st));
+  const size_t cbytes = sizeof(int) * (size_t)ntiles * nseg;
+  MRSR_TRY(counts.alloc(cbytes));
+  MRSR_TRY(total.alloc(sizeof(int) * ntiles));
+  MRSR_TRY(nch.alloc(sizeof(int) * ntiles));
+  MRSR_TRY(offset.alloc(sizeof(int) * ntiles));
+  MRSR_TRY(choff.alloc(sizeof(int) * ntiles));
+  MRSR_TRY(tile_of.alloc(sizeof(int) * std::max<int64_t>(S.n, 1)));
+  MRSR_TRY(order.alloc(sizeof(int) * std::max<int64_t>(S.n, 1)));
   MRSR_TRY(items.alloc(sizeof(int4) * maxitems));
-  MRSR_TRY(next.alloc(sizeof(int)));
-  const unsigned gt = (unsigned)std::max<int64_t>(cdiv(ntiles, 256), 1);
-  k_tile_items<<<gt, 256, 0, st>>>(counts.as<int>(), offset.as<int>(), choff.as<int>(), ntiles, items.as<int4>());
+  MRSR_TRY(nitems.alloc(sizeof(int)));
+  MRSR_TRY(next.alloc(sizeof(unsigned long long)));
+  MRSR_CHECK_CUDA(cudaMemsetAsync(counts.p, 0, cbytes, st));
+  const unsigned gb = (unsigned)std::min<int64_t>(std::max<int64_t>(cdiv(S.n, 256), 1), 152 * 16);
+  const unsigned gt = (unsigned)std::max<int64_t>(cdiv(ntiles, 64), 1);
+  k_tile_home<<<gb, 256, 0, st>>>(S, m0, m1, m2, tile, seg, ntiles, tile_of.as<int>(), counts.as<int>());
   MRSR_LAUNCH_CHECK();
+  k_tile_chunks<<<gt, 64, 0, st>>>(counts.as<int>(), nseg, ntiles, most, total.as<int>(), nch.as<int>());
+  MRSR_LAUNCH_CHECK();
+  k_tile_scan<<<1, 1024, 0, st>>>(total.as<int>(), nch.as<int>(), ntiles, offset.as<int>(), choff.as<int>(),
+                                  nitems.as<int>());
+  MRSR_LAUNCH_CHECK();
+  k_tile_items<<<gt, 64, 0, st>>>(counts.as<int>(), nseg, ntiles, most, offset.as<int>(), choff.as<int>(), items.as<int4>(),
+                                  big.as<int2>(), nbig.as<int>());
+  MRSR_LAUNCH_CHECK();
+  k_tile_scatter<<<gb, 256, 0, st>>>(S.n, seg, ntiles, tile_of.as<int>(), counts.as<int>(), order.as<int>());
+  MRSR_LAUNCH_CHECK();
+  if (stable) {
+    k_tile_order<<<152, 1024, 0, st>>>(big.as<int2>(), nbig.as<int>(), order.as<int>(), tmp.as<int>());
+    MRSR_LAUNCH_CHECK();
+  }
   return MRSR_OK;
 }
+
+constexpr int kTile3 = 8;                      // 3D interpolation windows
+constexpr int kWin3 = kTile3 + kEsWidth - 1;   // 15
+constexpr int kWin3Cells = kWin3 * kWin3 * kWin3;
 
 // 3D tap record: weights along x, y, z (the density compensation folded into wz), the
 // wrapped first tap, the linear sample index and its frame, in sorted order.
@@ -683,13 +727,7 @@ __global__ void k_tile_prep3(SampleSet S, int M0, int M1, int M2, const int* ord
     es_axis(k0, M0, r.wx, ix);
     es_axis(k1, M1, r.wy, iy);
     es_axis(k2, M2, r.wz, iz);
-    float w = 1.f;
-    if (dcf_kind == MRSR_DCF_RADIAL_3D || dcf_kind == MRSR_DCF_RADIAL_2D) {
-      const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(k0, k0), __fmul_rn(k1, k1)), __fmul_rn(k2, k2));
-      w = dcf_kind == MRSR_DCF_RADIAL_3D ? s2 : sqrtf(s2);
-    } else if (dcf_kind == MRSR_DCF_ARRAY) {
-      w = dcf[n];
-    }
+    const float w = sample_dcf(S, n, li, dcf_kind, dcf);
 #pragma unroll
     for (int j = 0; j < kEsWidth; ++j) r.wz[j] *= w;
     r.li = (int)li;
@@ -708,338 +746,20 @@ int TileSort::prep3(const SampleSet& S, int dcf_kind, const float* dcf, cudaStre
   const unsigned gb = (unsigned)std::min<int64_t>(std::max<int64_t>(cdiv(S.n, 256), 1), 152 * 16);
   k_tile_prep3<<<gb, 256, 0, st>>>(S, m0, m1, m2, order.as<int>(), dcf_kind, dcf, rec.as<TapRec3>());
   MRSR_LAUNCH_CHECK();
-  rec3 = true;
   return MRSR_OK;
 }
 
-struct TiledArgs {
-  SampleSet S;
-  int M0, M1;
-  int64_t cells;
-  int nparts;              // parts to spread (grid planes)
-  long long* q;            // [nparts][cells]
-  const FixedScale* fs;
-  int ntx;
-  const TapRec* rec;       // per-sample tap records in sorted order
-  const int4* items;       // (tile, first sorted position, count, -)
-  const int* nitems;
-  int* next;               // work counter, zeroed before the launch
-};
+}  // namespace mrsr
 
-// Part p of the Λ precompute: pair p0 + p / nq (k1 <= k2, packed k2 (k2 + 1) / 2 + k1), plane
-// p % nq; value conj(U[t,k1]) U[t,k2] 2^e (k_spread_lambda's value).
-struct LamParts {
-  const void* U;
-  int u_complex, nq, p0;
-  int64_t nt, ns_pf;
-  struct Lane {
-    int k1, k2, q;
-  };
-  __device__ Lane bind(int part) const {
-    const int ch = part / nq, q = part - ch * nq, p = p0 + ch;
-    int k2 = 0;
-    while ((k2 + 1) * (k2 + 2) / 2 <= p) ++k2;
-    return Lane{p - k2 * (k2 + 1) / 2, k2, q};
-  }
-  __device__ float value(const Lane& L, int64_t, int64_t t) const {
-    if (u_complex) {
-      const float2* u = reinterpret_cast<const float2*>(U);
-      const float2 v = cmulc(u[t + nt * L.k2], u[t + nt * L.k1]);  // conj(U[t,k1]) * U[t,k2]
-      return L.q ? v.y : v.x;
-    }
-    const float* u = reinterpret_cast<const float*>(U);
-    return u[t + nt * L.k2] * u[t + nt * L.k1];
-  }
-};
+#include "spread_rows.cuh"
 
-// Part p of the backprojection: channel p / 2 = (coil c0 + c) K + k, plane p % 2; value
-// y_c conj(U[t,k]) dcf (k_spread_data's value).
-struct DataParts {
-  const float2* data;
-  const void* U;
-  int u_complex, K, c0, dcf_kind;
-  const float* dcf;
-  int64_t nt, ns_pf, ns_tot;
-  struct Lane {
-    int c, k, q;
-  };
-  __device__ Lane bind(int part) const {
-    const int ch = part >> 1, c = ch / K;
-    return Lane{c, ch - c * K, part & 1};
-  }
-  __device__ float value(const Lane& L, int64_t li, int64_t t) const {
-    const float2 y = data[li + ns_tot * (c0 + L.c)];
-    float2 v;
-    if (u_complex) {
-      v = cmulc(y, reinterpret_cast<const float2*>(U)[t + nt * L.k]);  // y * conj(U)
-    } else {
-      const float uu = reinterpret_cast<const float*>(U)[t + nt * L.k];
-      v = make_float2(y.x * uu, y.y * uu);
-    }
-    return L.q ? v.y : v.x;
-  }
-};
-
-
-__device__ __noinline__ void spread_direct(long long* g, int M0, int M1, int lx0, int ly0, float v, const float* wx,
-                                           const float* wy) {
-  for (int t2 = 0; t2 < kEsWidth; ++t2) {
-    const int64_t row = (int64_t)M0 * wrap32(ly0 + t2, M1);
-    for (int t1 = 0; t1 < kEsWidth; ++t1)
-      atomicAdd(reinterpret_cast<unsigned long long*>(g + row + wrap32(lx0 + t1, M0)),
-                (unsigned long long)fx_term(v * wy[t2] * wx[t1]));
-  }
-}
-
-// Items are taken group-major (all tiles of part group 0, then group 1, ...) from a device
-// counter, so the CTAs in flight work on neighbouring tiles of one group and their flushes
-// share L2 lines.
-template <int P, class Parts>
-__global__ void __launch_bounds__(kTiledThreads, 2) k_spread_tiled(TiledArgs a, Parts parts) {
-  extern __shared__ __align__(16) int win[];  // [2][P][kWinCells]: low limbs, then high limbs
-  int* wlo = win;
-  int* whi = win + P * kWinCells;
-  __shared__ int s_item;
-  constexpr int SPW = 32 / P;  // samples per warp step
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int slot = lane / P, part = lane % P;
-  const int nitems = *a.nitems;
-  const int ngroups = (a.nparts + P - 1) / P;
-  const int total = nitems * ngroups;
-  const float sc = a.fs->scale;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(a.next, 1);
-    __syncthreads();
-    const int it = s_item;
-    if (it >= total) break;
-    const int grp = it / nitems;
-    const int4 item = a.items[it - grp * nitems];
-    const int gpart = grp * P + part;
-    const bool live_part = gpart < a.nparts;
-    const typename Parts::Lane L = parts.bind(live_part ? gpart : 0);
-    const int ox = (item.x % a.ntx) * kTile, oy = (item.x / a.ntx) * kTile;
-    int4* w4 = reinterpret_cast<int4*>(win);
-    for (int i = threadIdx.x; i < P * kWinCells / 2; i += blockDim.x) w4[i] = make_int4(0, 0, 0, 0);
-    __syncthreads();
-    for (int s0 = warp * SPW; s0 < item.z; s0 += nwarps * SPW) {
-      if (s0 + slot >= item.z || !live_part) continue;
-      const float4* r4 = reinterpret_cast<const float4*>(a.rec + item.y + s0 + slot);
-      float wx[kEsWidth], wy[kEsWidth];
-      {
-        const float4 q0 = r4[0], q1 = r4[1], q2 = r4[2], q3 = r4[3];
-        wx[0] = q0.x; wx[1] = q0.y; wx[2] = q0.z; wx[3] = q0.w;
-        wx[4] = q1.x; wx[5] = q1.y; wx[6] = q1.z; wx[7] = q1.w;
-        wy[0] = q2.x; wy[1] = q2.y; wy[2] = q2.z; wy[3] = q2.w;
-        wy[4] = q3.x; wy[5] = q3.y; wy[6] = q3.z; wy[7] = q3.w;
-      }
-      const int4 ri = reinterpret_cast<const int4*>(r4)[4];  // li, t, lx0, ly0
-      const float v = parts.value(L, ri.x, ri.y) * sc;
-      const int lx0 = ri.z, ly0 = ri.w;
-      const int lx = lx0 - ox, ly = ly0 - oy;
-      if ((unsigned)lx < (unsigned)kTile && (unsigned)ly < (unsigned)kTile) {
-        int* pl = wlo + part * kWinCells + ly * kWin + lx;
-        int* ph = whi + part * kWinCells + ly * kWin + lx;
-#pragma unroll
-        for (int t2 = 0; t2 < kEsWidth; ++t2) {
-          const float vy = v * wy[t2];
-#pragma unroll
-          for (int t1 = 0; t1 < kEsWidth; ++t1) {
-            int hi, lo;
-            fx_split_prod(vy, wx[t1], hi, lo);
-            atomicAdd(pl + t2 * kWin + t1, lo);
-            atomicAdd(ph + t2 * kWin + t1, hi);
-          }
-        }
-      } else {
-        // the sort put the first tap in this tile (the same float arithmetic); a sample
-        // outside it would go straight to the grid rather than out of the window
-        spread_direct(a.q + (int64_t)gpart * a.cells, a.M0, a.M1, lx0, ly0, v, wx, wy);
-      }
-    }
-    __syncthreads();
-    const int gx = wrap32(ox + lane, a.M0);
-    for (int task = warp; task < P * kWin; task += nwarps) {
-      const int p = task / kWin, row = task - p * kWin;
-      const int gp = grp * P + p;
-      if (gp >= a.nparts || lane >= kWin) continue;
-      const int c = p * kWinCells + row * kWin + lane;
-      const long long v = (long long)whi[c] * (1ll << kFxLoBits) + (long long)wlo[c];
-      if (v != 0)
-        atomicAdd(reinterpret_cast<unsigned long long*>(a.q + (int64_t)gp * a.cells + gx +
-                                                        (int64_t)a.M0 * wrap32(oy + row, a.M1)),
-                  (unsigned long long)v);
-    }
-    __syncthreads();
-  }
-}
-
-template <int P, class Parts>
-static int launch_tiled(const TiledArgs& a, const Parts& parts, cudaStream_t st) {
-  constexpr int smem = tiled_smem_bytes<P>();
-  MRSR_CHECK_CUDA(cudaFuncSetAttribute(k_spread_tiled<P, Parts>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  MRSR_CHECK_CUDA(cudaMemsetAsync(a.next, 0, sizeof(int), st));
-  k_spread_tiled<P, Parts><<<152 * 2, kTiledThreads, smem, st>>>(a, parts);
-  MRSR_LAUNCH_CHECK();
-  return MRSR_OK;
-}
-
-template <class Parts>
-static int spread_tiled(const SampleSet& S, const int64_t* M, int64_t cells, int nparts, long long* q,
-                        const FixedScale* fs, const TileSort& ts, const Parts& parts, cudaStream_t st) {
-  MRSR_REQUIRE(ts.m0 == (int)M[0] && ts.m1 == (int)M[1], MRSR_ERR_STATE, "tile sort built for another grid");
-  MRSR_REQUIRE(ts.rec.p != nullptr, MRSR_ERR_STATE, "tile sort without tap records");
-  const TiledArgs a{S, ts.m0, ts.m1, cells, nparts, q, fs, ts.ntx,
-                    ts.rec.as<TapRec>(), ts.items.as<int4>(), ts.nitems.as<int>(), ts.next.as<int>()};
-  return nparts <= 16 ? launch_tiled<16>(a, parts, st) : launch_tiled<32>(a, parts, st);
-}
-
-// ------------------------------------------------- tile-sorted (3D) ---
-//
-// The 2D scheme in three dimensions: samples in 8^3 tiles (home tile of the first tap), work
-// items of at most kChunk samples of one tile x a group of kP3 = 4 parts, a window of
-// (8 + w - 1)^3 = 15^3 cells x 4 parts of 32-bit limbs in shared memory (106 KB: two CTAs
-// per SM), and one global 64-bit atomic per nonzero window cell at the flush, a warp on
-// consecutive cells.  A warp takes one sample at a time: lane = 8 part + t1 (part < 4, x tap
-// t1 < 8), so a warp instruction adds 8 consecutive cells of 4 parts, and the part stride
-// (3384 = 24 mod 32 words) puts the four 8-cell runs in disjoint bank ranges: no bank
-// conflicts.  With 64-bit global atomics capped near 0.73 T/s on this GPU, every term as a
-// global atomic (the one-warp-per-sample kernels) spends ~0.55 s on the 401 G terms of a
-// 128^3, 4.9 M-sample, 16-coil backprojection.
-constexpr int kWin3 = kTile3 + kEsWidth - 1;           // 15
-constexpr int kWin3Cells = kWin3 * kWin3 * kWin3;      // 3375
-constexpr int kWin3Stride = 3384;                      // part stride, = 24 (mod 32)
-constexpr int kP3 = 4;
-constexpr int kTiled3Smem = 2 * kP3 * kWin3Stride * (int)sizeof(int);
-static_assert(kWin3Stride >= kWin3Cells && kWin3Stride % 32 == 24 && kWin3Stride % 4 == 0, "3D window stride");
-
-struct TiledArgs3 {
-  SampleSet S;
-  int M0, M1, M2;
-  int64_t cells;
-  int nparts;
-  long long* q;            // [nparts][cells]
-  const FixedScale* fs;
-  int ntx, nty;
-  const TapRec3* rec;
-  const int4* items;
-  const int* nitems;
-  int* next;
-};
-
-template <class Parts>
-__global__ void __launch_bounds__(kTiledThreads, 2) k_spread_tiled3(TiledArgs3 a, Parts parts) {
-  extern __shared__ __align__(16) int win3[];  // [2][kP3][kWin3Stride]
-  int* wlo = win3;
-  int* whi = win3 + kP3 * kWin3Stride;
-  __shared__ int s_item;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int part = lane >> 3, t1 = lane & 7;
-  const int nitems = *a.nitems;
-  const int ngroups = (a.nparts + kP3 - 1) / kP3;
-  const int total = nitems * ngroups;
-  const float sc = a.fs->scale;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(a.next, 1);
-    __syncthreads();
-    const int it = s_item;
-    if (it >= total) break;
-    const int grp = it / nitems;
-    const int4 item = a.items[it - grp * nitems];
-    const int gpart = grp * kP3 + part;
-    const bool live_part = gpart < a.nparts;
-    const typename Parts::Lane L = parts.bind(live_part ? gpart : 0);
-    const int tx = item.x % a.ntx, tyz = item.x / a.ntx;
-    const int ox = tx * kTile3, oy = (tyz % a.nty) * kTile3, oz = (tyz / a.nty) * kTile3;
-    int4* w4 = reinterpret_cast<int4*>(win3);
-    for (int i = threadIdx.x; i < 2 * kP3 * kWin3Stride / 4; i += blockDim.x) w4[i] = make_int4(0, 0, 0, 0);
-    __syncthreads();
-    if (live_part) {
-      for (int smp = warp; smp < item.z; smp += nwarps) {
-        const float4* r4 = reinterpret_cast<const float4*>(a.rec + item.y + smp);
-        float wy[kEsWidth], wz[kEsWidth];
-        {
-          const float4 q2 = r4[2], q3 = r4[3], q4 = r4[4], q5 = r4[5];
-          wy[0] = q2.x; wy[1] = q2.y; wy[2] = q2.z; wy[3] = q2.w;
-          wy[4] = q3.x; wy[5] = q3.y; wy[6] = q3.z; wy[7] = q3.w;
-          wz[0] = q4.x; wz[1] = q4.y; wz[2] = q4.z; wz[3] = q4.w;
-          wz[4] = q5.x; wz[5] = q5.y; wz[6] = q5.z; wz[7] = q5.w;
-        }
-        const float wx1 = reinterpret_cast<const float*>(r4)[t1];
-        const int4 ri = reinterpret_cast<const int4*>(r4)[6];  // li, t, lx0, ly0
-        const int lz0 = reinterpret_cast<const int*>(r4)[28];
-        const float v = parts.value(L, ri.x, ri.y) * sc * wx1;
-        const int lx = ri.z - ox, ly = ri.w - oy, lz = lz0 - oz;
-        if ((unsigned)lx < (unsigned)kTile3 && (unsigned)ly < (unsigned)kTile3 && (unsigned)lz < (unsigned)kTile3) {
-          const int base = part * kWin3Stride + (lz * kWin3 + ly) * kWin3 + lx + t1;
-          int* pl = wlo + base;
-          int* ph = whi + base;
-#pragma unroll
-          for (int t3 = 0; t3 < kEsWidth; ++t3) {
-            const float v3 = v * wz[t3];
-#pragma unroll
-            for (int t2 = 0; t2 < kEsWidth; ++t2) {
-              int hi, lo;
-              fx_split_prod(v3, wy[t2], hi, lo);
-              atomicAdd(pl + (t3 * kWin3 + t2) * kWin3, lo);
-              atomicAdd(ph + (t3 * kWin3 + t2) * kWin3, hi);
-            }
-          }
-        } else {
-          // the sort put the first tap in this tile (the same float arithmetic); a sample
-          // outside it goes straight to the grid rather than out of the window
-          long long* g = a.q + (int64_t)gpart * a.cells;
-          const int64_t x = wrap32(ri.z + t1, a.M0);
-          for (int t3 = 0; t3 < kEsWidth; ++t3)
-            for (int t2 = 0; t2 < kEsWidth; ++t2) {
-              const int64_t row = (int64_t)a.M0 * (wrap32(ri.w + t2, a.M1) + (int64_t)a.M1 * wrap32(lz0 + t3, a.M2));
-              atomicAdd(reinterpret_cast<unsigned long long*>(g + row + x),
-                        (unsigned long long)fx_term(v * wz[t3] * wy[t2]));
-            }
-        }
-      }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < kP3 * kWin3Cells; e += blockDim.x) {
-      const int p = e / kWin3Cells, c = e - p * kWin3Cells;
-      const int gp = grp * kP3 + p;
-      if (gp >= a.nparts) continue;
-      const int w = p * kWin3Stride + c;
-      const long long v = (long long)whi[w] * (1ll << kFxLoBits) + (long long)wlo[w];
-      if (v == 0) continue;
-      const int cx = c % kWin3, cyz = c / kWin3;
-      const int cy = cyz % kWin3, cz = cyz / kWin3;
-      const int64_t cell = wrap32(ox + cx, a.M0) +
-                           (int64_t)a.M0 * (wrap32(oy + cy, a.M1) + (int64_t)a.M1 * wrap32(oz + cz, a.M2));
-      atomicAdd(reinterpret_cast<unsigned long long*>(a.q + (int64_t)gp * a.cells + cell), (unsigned long long)v);
-    }
-    __syncthreads();
-  }
-}
-
-template <class Parts>
-static int spread_tiled3(const SampleSet& S, const int64_t* M, int64_t cells, int nparts, long long* q,
-                         const FixedScale* fs, const TileSort& ts, const Parts& parts, cudaStream_t st) {
-  MRSR_REQUIRE(ts.rec3 && ts.m0 == (int)M[0] && ts.m1 == (int)M[1] && ts.m2 == (int)M[2], MRSR_ERR_STATE,
-               "3D tile sort built for another grid or without tap records");
-  const TiledArgs3 a{S, ts.m0, ts.m1, ts.m2, cells, nparts, q, fs, ts.ntx, ts.nty,
-                     ts.rec.as<TapRec3>(), ts.items.as<int4>(), ts.nitems.as<int>(), ts.next.as<int>()};
-  MRSR_CHECK_CUDA(cudaFuncSetAttribute(k_spread_tiled3<Parts>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kTiled3Smem));
-  MRSR_CHECK_CUDA(cudaMemsetAsync(a.next, 0, sizeof(int), st));
-  k_spread_tiled3<Parts><<<152 * 2, kTiledThreads, kTiled3Smem, st>>>(a, parts);
-  MRSR_LAUNCH_CHECK();
-  return MRSR_OK;
-}
+namespace mrsr {
 
 int spread_lambda(const SpreadLambdaArgs& a, const TileSort* ts, cudaStream_t st) {
   if (a.S.n == 0) return MRSR_OK;
-  if (ts && a.S.d == 2) {
-    const LamParts parts{a.U, a.u_complex, a.nq, a.p0, a.S.nt, a.S.ns_pf};
-    return spread_tiled(a.S, a.M, a.cells, a.np * a.nq, a.q, a.fs, *ts, parts, st);
-  }
-  if (ts && a.S.d == 3 && ts->rec3) {
-    const LamParts parts{a.U, a.u_complex, a.nq, a.p0, a.S.nt, a.S.ns_pf};
-    return spread_tiled3(a.S, a.M, a.cells, a.np * a.nq, a.q, a.fs, *ts, parts, st);
+  if (ts && ts->rec.p) {
+    const LamParts parts{a.U, a.umax, a.u_complex, a.nq, a.p0, a.S.nt};
+    return spread_rows(a.S.d, a.M, a.cells, a.np * a.nq, a.q, a.fs, *ts, parts, st);
   }
   MRSR_REQUIRE(a.cells < (1ll << 32), MRSR_ERR_UNSUPPORTED, "spreading grid of 2^32 cells or more");
   const int* order = ts ? ts->order.as<int>() : nullptr;
@@ -1053,11 +773,14 @@ int spread_lambda(const SpreadLambdaArgs& a, const TileSort* ts, cudaStream_t st
 
 int spread_data(const SpreadDataArgs& a, const TileSort* ts, cudaStream_t st) {
   if (a.S.n == 0) return MRSR_OK;
-  if (ts && a.U && (a.S.d == 2 || ts->rec3)) {
-    const DataParts parts{a.data, a.U, a.u_complex, a.K, a.c0, a.dcf_kind, a.dcf,
-                          a.S.nt, a.S.ns_pf, a.S.ns_pf * a.S.nt};
-    if (a.S.d == 2) return spread_tiled(a.S, a.M, a.cells, 2 * a.nc * a.K, a.q, a.fs, *ts, parts, st);
-    return spread_tiled3(a.S, a.M, a.cells, 2 * a.nc * a.K, a.q, a.fs, *ts, parts, st);
+  if (ts && a.U && ts->rec.p) {
+    const unsigned gb = (unsigned)std::min<int64_t>(cdiv(a.S.n, 256), 152 * 16);
+    MRSR_CHECK_CUDA(cudaMemsetAsync(a.tmax, 0, sizeof(float) * (size_t)ts->ntiles * a.nc, st));
+    k_tile_absmax<<<gb, 256, 0, st>>>(a.S, ts->tile_of.as<int>(), a.data, a.c0, a.nc, a.dcf_kind, a.dcf,
+                                      reinterpret_cast<unsigned*>(a.tmax));
+    MRSR_LAUNCH_CHECK();
+    const DataParts parts{a.data, a.U, a.umax, a.tmax, a.u_complex, a.K, a.c0, a.nc, a.S.nt, a.S.ns_pf * a.S.nt};
+    return spread_rows(a.S.d, a.M, a.cells, 2 * a.nc * a.K, a.q, a.fs, *ts, parts, st);
   }
   MRSR_REQUIRE(a.cells < (1ll << 32), MRSR_ERR_UNSUPPORTED, "spreading grid of 2^32 cells or more");
   const int* order = ts && a.S.d == 3 ? ts->order.as<int>() : nullptr;
@@ -1113,17 +836,11 @@ int fixed_scale(const float* const* f, const int64_t* n, int nf, double mult, do
   return MRSR_OK;
 }
 
-// int64 -> float32 without the float64 pipe: v = hi * 2^32 + lo with lo in [-2^31, 2^31)
-// (so a small negative v is lo alone, with no cancellation), each half converted in float32
-// and joined by one fma (within ~2 float32 roundings of v), then scaled by 2^-e
+// fixed-point planes -> float2 grids
 __global__ void k_fixed_to_grid(const long long* q, int nq, int64_t cells, int64_t total, const FixedScale* fs,
                                 float2* out) {
   const float inv = fs->inv;
-  auto cvt = [inv](long long v) {
-    const long long hi = (v + (1ll << 31)) >> 32;
-    const int lo = (int)(v - hi * 4294967296ll);
-    return __fmaf_rn((float)(int)hi, 4294967296.f, (float)lo) * inv;
-  };
+  auto cvt = [inv](long long v) { return fx_to_float(v) * inv; };
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t ch = e / cells, cell = e - ch * cells;
     const long long* qc = q + ch * nq * cells + cell;
@@ -1282,15 +999,17 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   MRSR_TRY(fG.init(d, G));
   const float* ipsi[3] = {nullptr, nullptr, nullptr};
   for (int i = 0; i < d; ++i) MRSR_TRY(es_inv_psi_table(M[i], -G[i] / 2, G[i] + 1, &ipsi[i]));
-  // channel batches of ~2 GB of upsampled float2 grid; the 3D tile-sorted kernel takes four
-  // parts per pass, so a 3D batch holds at least four channels' parts (8-12 GB on 512^3)
+  // channel batches of ~2 GB of upsampled float2 grid; the tile-sorted kernel takes at least
+  // eight parts per pass, so a 3D batch holds that many (8 GB each of float2 and fixed-point grid on 512^3)
   const int nq = u_complex ? 2 : 1;  // a real basis spreads real values
   const int64_t max_bytes = 2ll << 30;
   int pb = (int)std::max<int64_t>(1, std::min<int64_t>(P, max_bytes / (mcells * (int64_t)sizeof(float2))));
-  if (d == 3) pb = std::max(pb, std::min(P, kP3 / nq));
-  DevBuf grid, qgrid, cgrid, fsb;
+  if (d == 3) pb = std::max(pb, std::min(P, 8 / nq));
+  const bool tiled = S.n < (1ll << 31) && S.ns_pf * S.nt < (1ll << 31);
+  DevBuf grid, qgrid, cgrid, fsb, umax;
+  const size_t qbytes = tiled ? spread_rows_bytes(nq * pb, mcells) : sizeof(long long) * nq * mcells * pb;
   MRSR_TRY(grid.alloc(sizeof(float2) * mcells * pb));
-  MRSR_TRY(qgrid.alloc(sizeof(long long) * nq * mcells * pb));
+  MRSR_TRY(qgrid.alloc(qbytes));
   MRSR_TRY(cgrid.alloc(sizeof(float2) * gcells * P));
   // fixed-point scale: |term| <= (2 if complex) max|U|^2 (the kernel taps are <= 1), and a cell
   // of the upsampled grid gets at most ceil(w / M) taps per sample and dimension
@@ -1303,25 +1022,27 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
     MRSR_TRY(fixed_scale(f, n, 2, u_complex ? 2.0 : 1.0, (double)S.n * taps_per_cell(d, M), fsb.as<FixedScale>(), st));
   }
   TileSort ts;
-  const bool tiled = d == 2 && S.ns_pf * S.nt < (1ll << 31);
-  const bool ordered = d == 3 && S.n < (1ll << 31);
+  const bool ordered = S.n < (1ll << 31) && d == 3;
+  if (tiled || ordered) MRSR_TRY(ts.build(S, M, kSpTile, kSpChunk, true, st));
   if (tiled) {
-    MRSR_TRY(ts.build(S, M[0], M[1], st));
     MRSR_TRY(ts.prep(S, MRSR_DCF_NONE, nullptr, st));
-  } else if (ordered) {
-    MRSR_TRY(ts.build3(S, M, st));
-    if (S.ns_pf * S.nt < (1ll << 31)) MRSR_TRY(ts.prep3(S, MRSR_DCF_NONE, nullptr, st));
+    MRSR_TRY(umax.alloc(sizeof(float) * K));
+    k_basis_max<<<K, 256, 0, st>>>(U, S.nt, u_complex, umax.as<float>());
+    MRSR_LAUNCH_CHECK();
   }
   const TileSort* tsp = tiled || ordered ? &ts : nullptr;
   MRSR_TRY(packed.alloc((u_complex ? 8 : 4) * (size_t)P * std::max<int64_t>(*nk_out, 1)));
   // channels in batches of pb: spread, inverse DFT on the upsampled grid, deconvolve and fold onto the 2x grid
   for (int p0 = 0; p0 < P; p0 += pb) {
     const int np = std::min(pb, P - p0);
-    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, sizeof(long long) * nq * mcells * np, st));
+    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, tiled ? spread_rows_bytes(nq * np, mcells) : sizeof(long long) * nq * mcells * np, st));
     SpreadLambdaArgs sa{S, {M[0], M[1], M[2]}, mcells, U, u_complex, K, P, p0, np, nq, qgrid.as<long long>(),
-                        fsb.as<FixedScale>()};
+                        fsb.as<FixedScale>(), umax.as<float>()};
     MRSR_TRY(spread_lambda(sa, tsp, st));
-    MRSR_TRY(fixed_to_grid(qgrid.as<long long>(), nq, mcells, np, fsb.as<FixedScale>(), grid.as<float2>(), st));
+    if (tiled)
+      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), nq, mcells, nq * np, fsb.as<FixedScale>(), grid.as<float2>(), st));
+    else
+      MRSR_TRY(fixed_to_grid(qgrid.as<long long>(), nq, mcells, np, fsb.as<FixedScale>(), grid.as<float2>(), st));
     MRSR_TRY(fM.run(grid.as<float2>(), np, +1, 1.0f, st));
     FoldArgs fa;
     fa.d = d;
@@ -1814,17 +1535,17 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
   int cc = (int)std::max<int64_t>(1, std::min<int64_t>(ncoils, max_bytes / std::max<int64_t>(per_coil, 1)));
   // 3D with a basis: the batch's parts (2 per coil and coefficient) interleaved per cell, at
   // most 32 (one per lane of k_spread_data_cp)
-  const bool tiled3 = ndims == 3 && U != nullptr && sl.set.n < (1ll << 31) && ns_per_frame * nt < (1ll << 31);
-  const bool parts_layout = ndims == 3 && U != nullptr && !tiled3 && 2 * K <= 32;
+  const bool tiled = U != nullptr && sl.set.n < (1ll << 31) && ns_per_frame * nt < (1ll << 31);
+  const bool parts_layout = ndims == 3 && U != nullptr && !tiled && 2 * K <= 32;
   if (parts_layout) cc = std::min(cc, 16 / K);
   DevBuf grid, qgrid, fsb;
   MRSR_TRY(grid.alloc((size_t)per_coil * cc));
-  MRSR_TRY(qgrid.alloc((size_t)per_coil * 2 * cc));  // fixed-point re and im, 8 bytes each
+  // fixed-point re and im, 8 bytes each
+  MRSR_TRY(qgrid.alloc(tiled ? spread_rows_bytes(2 * K * cc, mcells) : (size_t)per_coil * 2 * cc));
   // fixed-point scale: |term component| <= max|data| max|U| (x2 for complex U) x dcf bound,
   // at most ceil(w / M) taps per sample, cell and dimension
   MRSR_TRY(fsb.alloc(sizeof(FixedScale)));
   // an identity basis gives every sample one channel: the global kernel
-  const bool tiled = ndims == 2 && U != nullptr && ns_per_frame * nt < (1ll << 31);
   {
     const float* f[3];
     int64_t n[3];
@@ -1846,22 +1567,28 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
     MRSR_TRY(fixed_scale(f, n, nf, mult, (double)sl.set.n * taps_per_cell(ndims, M), fsb.as<FixedScale>(), st));
   }
   TileSort ts;
-  if (tiled) {
-    MRSR_TRY(ts.build(sl.set, M[0], M[1], st));
-    MRSR_TRY(ts.prep(sl.set, dcf_kind, dcf_array, st));
-  }
+  DevBuf umax, tmax;
   const bool ordered = ndims == 3 && sl.set.n < (1ll << 31);
-  if (ordered) MRSR_TRY(ts.build3(sl.set, M, st));
-  if (tiled3) MRSR_TRY(ts.prep3(sl.set, dcf_kind, dcf_array, st));
+  if (tiled || ordered) MRSR_TRY(ts.build(sl.set, M, kSpTile, kSpChunk, true, st));
+  if (tiled) {
+    MRSR_TRY(ts.prep(sl.set, dcf_kind, dcf_array, st));
+    MRSR_TRY(umax.alloc(sizeof(float) * K));
+    MRSR_TRY(tmax.alloc(sizeof(float) * (size_t)ts.ntiles * cc));
+    k_basis_max<<<K, 256, 0, st>>>(U, nt, u_is_complex, umax.as<float>());
+    MRSR_LAUNCH_CHECK();
+  }
   const int64_t out_elems = nimg * K * (cmaps ? 1 : ncoils);
   if (cmaps) MRSR_CHECK_CUDA(cudaMemsetAsync(out, 0, sizeof(float2) * out_elems, st));
   for (int c0 = 0; c0 < ncoils; c0 += cc) {
     const int nc = std::min(cc, ncoils - c0);
-    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, (size_t)per_coil * 2 * nc, st));
+    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, tiled ? spread_rows_bytes(2 * K * nc, mcells) : (size_t)per_coil * 2 * nc, st));
     SpreadDataArgs sa{sl.set, {M[0], M[1], M[2]}, mcells, reinterpret_cast<const float2*>(data), c0, nc, U,
-                      u_is_complex, K, dcf_kind, dcf_array, qgrid.as<long long>(), fsb.as<FixedScale>()};
+                      u_is_complex, K, dcf_kind, dcf_array, qgrid.as<long long>(), fsb.as<FixedScale>(), umax.as<float>(),
+                      tmax.as<float>()};
     MRSR_TRY(spread_data(sa, tiled || ordered ? &ts : nullptr, st));
-    if (parts_layout) {
+    if (tiled) {
+      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), 2, mcells, 2 * K * nc, fsb.as<FixedScale>(), grid.as<float2>(), st));
+    } else if (parts_layout) {
       k_fixed_to_grid_cp<<<(unsigned)cdiv(mcells, 32), 256, 0, st>>>(qgrid.as<long long>(), 2 * nc * K, mcells,
                                                                     fsb.as<FixedScale>(), grid.as<float2>());
       MRSR_LAUNCH_CHECK();
@@ -1926,11 +1653,11 @@ extern "C" int mrsr_forward_model(int ndims, const int64_t* img_shape, int64_t n
   const int64_t ntiles3 = cdiv(M[0], kTile3) * cdiv(M[1], kTile3) * cdiv(M[2], kTile3);
   const bool tiled3 = ndims == 3 && small && ntiles3 < (1ll << 31) && mcells < (1ll << 32);
   if (tiled) {
-    MRSR_TRY(ts.build(sl.set, M[0], M[1], st));
+    MRSR_TRY(ts.build(sl.set, M, kTile, kChunk, false, st));
     MRSR_TRY(ts.prep(sl.set, MRSR_DCF_NONE, nullptr, st));
   } else if (tiled3) {
-    MRSR_TRY(ts.build3(sl.set, M, st));
-    MRSR_TRY(ts.prep3(sl.set, MRSR_DCF_NONE, nullptr, st));
+    MRSR_TRY(ts.build(sl.set, M, kTile3, kChunk, false, st));
+    MRSR_TRY(ts.prep(sl.set, MRSR_DCF_NONE, nullptr, st));
   }
   const size_t win_bytes = sizeof(float2) * kWinCells * (size_t)K;
   const size_t win3_bytes = sizeof(float2) * kWin3Cells * (size_t)K;

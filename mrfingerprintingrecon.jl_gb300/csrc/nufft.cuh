@@ -100,20 +100,19 @@ __device__ __forceinline__ void fx_split(float a, int& hi, int& lo) {
   lo = __float_as_int(__fmaf_rn(d, (float)(1 << kFxLoBits), kMagic)) - kMagicBits;  // |lo| <= 2^20
 }
 
-// fx_split of the product a = x * y, the first rounding fused into the product
-__device__ __forceinline__ void fx_split_prod(float x, float y, int& hi, int& lo) {
-  constexpr float kMagic = 12582912.f;
-  constexpr int kMagicBits = 0x4B400000;
-  const float s1 = __fmaf_rn(x, y, kMagic);
-  hi = __float_as_int(s1) - kMagicBits;                          // round(x y)
-  const float d = __fmaf_rn(x, y, -__fsub_rn(s1, kMagic));       // x y - round(x y), |d| <= 1/2
-  lo = __float_as_int(__fmaf_rn(d, (float)(1 << kFxLoBits), kMagic)) - kMagicBits;
-}
-
 __device__ __forceinline__ long long fx_term(float a) {
   int hi, lo;
   fx_split(a, hi, lo);
   return (long long)hi * (1ll << kFxLoBits) + lo;
+}
+
+// int64 -> float32 without the float64 pipe: v = hi * 2^32 + lo with lo in [-2^31, 2^31)
+// (so a small negative v is lo alone, with no cancellation), each half converted in float32
+// and joined by one fma (within ~2 float32 roundings of v)
+__device__ __forceinline__ float fx_to_float(long long v) {
+  const long long hi = (v + (1ll << 31)) >> 32;
+  const int lo = (int)(v - hi * 4294967296ll);
+  return __fmaf_rn((float)(int)hi, 4294967296.f, (float)lo);
 }
 
 // grid[ch][part][cell] (part: re, and im for complex grids) += value(ch, n) * phi taps,
@@ -127,30 +126,27 @@ struct SpreadLambdaArgs {
   int P;              // channels: packed pairs k1 <= k2
   int p0, np;         // spread only channels p0 .. p0+np-1
   int nq;             // parts per cell: 1 (real basis: the spread values are real) or 2
-  long long* q;       // [np][nq][cells]
+  long long* q;       // [np][nq][cells], or the parts layout of spread_rows.cuh with tap records
   const FixedScale* fs;
+  const float* umax;  // with tap records: k_basis_max of U
 };
-// Samples of a 2D set counting-sorted by the 12 x 12 tile of the grid M0 x M1 that holds
-// their first tap, in chunks of at most 1024 samples (the work items of the tile-sorted
-// spreading kernels).  Built once per sample set and grid, shared by every spread of it.
-// build3: for a 3D set, `order` and work items by 8 x 8 x 8 tiles (the global kernels take
-// samples in that order, so the warps in flight touch neighbouring grid lines in L2; the
-// 3D tile-sorted kernel takes the items).
-// prep: the per-sample tap records the 2D tile-sorted kernels read (weights with the
-// density compensation folded in, first tap, sample index and frame), after build.
-// prep3: the same records for the 3D tile-sorted kernels, after build3.
+// Samples of a set counting-sorted by the tile (`tile` cells a side) of the grid M that holds
+// their first tap, in chunks (the work items of the tile-sorted kernels) of at most `most`
+// samples; with `stable`, which samples a chunk holds does not change from run to run.  Built once per sample set and grid, shared by every spread of it; the global 3D
+// kernels take samples in that order too, so the warps in flight touch neighbouring grid lines.
+// prep: the per-sample tap records the tile-sorted kernels read (weights with the density
+// compensation folded in, first tap, sample index and frame), after build.
 struct TileSort {
-  DevBuf counts, offset, choff, cursor, tile_of, order, items, nitems, next, rec;
-  int ntx = 0, nty = 0, ntiles = 0, m0 = 0, m1 = 0, m2 = 0;
-  bool rec3 = false;
-  int build(const SampleSet& S, int64_t M0, int64_t M1, cudaStream_t st);
-  int build3(const SampleSet& S, const int64_t* M, cudaStream_t st);
+  DevBuf counts, total, nch, offset, choff, tile_of, order, items, nitems, next, rec;
+  int tile = 0, ntx = 0, nty = 0, ntiles = 0, m0 = 0, m1 = 0, m2 = 0;
+  int build(const SampleSet& S, const int64_t* M, int tile, int most, bool stable, cudaStream_t st);
   int prep(const SampleSet& S, int dcf_kind, const float* dcf, cudaStream_t st);
+ private:
   int prep3(const SampleSet& S, int dcf_kind, const float* dcf, cudaStream_t st);
 };
 
-// ts: tile sort of a.S on a.M.  2D: the tile-sorted kernel; 3D (ts from build3, or null):
-// the global kernel (one warp per sample, every term a global atomic).
+// ts: tile sort of a.S on a.M with tap records: the tile-sorted kernel; without records, or
+// null: the global kernel (one warp per sample, every term a global atomic).
 int spread_lambda(const SpreadLambdaArgs& a, const TileSort* ts, cudaStream_t st);
 
 struct SpreadDataArgs {
@@ -162,8 +158,10 @@ struct SpreadDataArgs {
   int u_complex, K;
   int dcf_kind;
   const float* dcf;     // per kept sample (dcf_kind == array)
-  long long* q;         // [(c - c0) * K + k][2][cells]
+  long long* q;         // [(c - c0) * K + k][2][cells], or the parts layout of spread_rows.cuh with tap records
   const FixedScale* fs;
+  const float* umax;    // with tap records: k_basis_max of U, and room for ntiles * nc maxima
+  float* tmax;
 };
 int spread_data(const SpreadDataArgs& a, const TileSort* ts, cudaStream_t st);
 
