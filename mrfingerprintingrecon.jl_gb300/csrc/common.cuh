@@ -49,15 +49,13 @@ struct Status {
 // Every entry point that takes a stream opens a CallScope on it.  Device
 // memory comes from the stream-ordered pool (cudaMallocAsync) on the call's
 // stream, so the library never calls cudaMalloc / cudaFree, which would
-// synchronise the whole device and stall other streams' work.  A buffer is
-// freed on the library's private stream after that stream has waited for the
-// work that may still use it: the running call's stream (temporaries) or the
-// owning operator's last use (see mrsr_normalop).
+// synchronise the whole device and stall other streams' work.  A buffer released
+// inside a call is freed on the call's stream; one released with its operator, on
+// the library's private stream after that stream has waited for the operator's
+// last use (see mrsr_normalop).
 cudaStream_t lib_stream();          // private non-blocking stream of the current device
 cudaStream_t call_stream();         // stream of the running entry point, else lib_stream()
 bool in_call();
-// lib_stream() waits for the work enqueued so far on `s`
-int fence_lib_after(cudaStream_t s);
 // host -> device copy ordered on call_stream() (pageable source may be freed on return)
 int copy_h2d(void* dst, const void* src, size_t bytes);
 

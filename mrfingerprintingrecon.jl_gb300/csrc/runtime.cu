@@ -10,7 +10,6 @@ namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 cudaStream_t g_lib[kMaxDevices] = {nullptr};
-cudaEvent_t g_fence[kMaxDevices] = {nullptr};
 thread_local cudaStream_t t_call = nullptr;
 thread_local bool t_in_call = false;
 
@@ -25,7 +24,6 @@ int current_device() {
 // to hand a block over
 void init_device(int d) {
   cudaStreamCreateWithFlags(&g_lib[d], cudaStreamNonBlocking);
-  cudaEventCreateWithFlags(&g_fence[d], cudaEventDisableTiming);
   cudaMemPool_t pool;
   if (cudaDeviceGetDefaultMemPool(&pool, d) == cudaSuccess) {
     uint64_t keep = 8ull << 30;
@@ -46,16 +44,6 @@ cudaStream_t lib_stream() {
 cudaStream_t call_stream() { return t_in_call ? t_call : lib_stream(); }
 bool in_call() { return t_in_call; }
 
-int fence_lib_after(cudaStream_t s) {
-  cudaStream_t ls = lib_stream();
-  if (s == ls) return MRSR_OK;
-  const int d = current_device();
-  std::lock_guard<std::mutex> lock(g_mu);  // one fence event per device, reused under the lock
-  MRSR_CHECK_CUDA(cudaEventRecord(g_fence[d], s));
-  MRSR_CHECK_CUDA(cudaStreamWaitEvent(ls, g_fence[d], 0));
-  return MRSR_OK;
-}
-
 int copy_h2d(void* dst, const void* src, size_t bytes) {
   cudaStream_t s = call_stream();
   MRSR_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
@@ -72,11 +60,12 @@ CallScope::~CallScope() {
   t_in_call = prev_in;
 }
 
+// Inside a call the block goes back on the call's own stream: the next call on that stream
+// takes it again without waiting for it (freed on another stream, it is out of reach until the
+// GPU has got there, and calls in a row without a synchronisation made the pool grow).
 void DevBuf::release() {
   if (!p) return;
-  cudaStream_t ls = lib_stream();
-  if (t_in_call) fence_lib_after(t_call);
-  cudaFreeAsync(p, ls);
+  cudaFreeAsync(p, t_in_call ? t_call : lib_stream());
   p = nullptr;
   bytes = 0;
 }
@@ -84,6 +73,7 @@ void DevBuf::release() {
 int DevBuf::alloc(size_t n) {
   release();
   if (n == 0) return MRSR_OK;
+  lib_stream();  // sets the device's pool up on first use
   cudaStream_t s = call_stream();
   cudaError_t e = cudaMallocAsync(&p, n, s);
   if (e == cudaSuccess && !t_in_call) e = cudaStreamSynchronize(s);
