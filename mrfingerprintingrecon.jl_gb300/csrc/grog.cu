@@ -7,9 +7,10 @@
 // matrices accumulated in float64, Gauss-Jordan with partial pivoting); the
 // principal matrix logarithm runs in float32, the precision the reference
 // computes log(G) in, by inverse scaling and squaring: Denman-Beavers square
-// roots until ||Y - I||_F <= 1/4, then log(I + X) by the m-point Gauss-Legendre
-// quadrature of int_0^1 X (I + t X)^{-1} dt (the diagonal Pade approximant),
-// times 2^s (Higham, Functions of Matrices, SIAM 2008, ch. 11).
+// roots until ||Y - I||_F <= 0.8, then log(Y) = 2 atanh((Y - I)(Y + I)^{-1}) by
+// its power series, times 2^s (Higham, Functions of Matrices, SIAM 2008, ch. 11).
+// (A quadrature that needed ||Y - I||_F <= 1/4 took one or two more square roots,
+// whose roundings 2^s multiplies, and twelve more inversions.)
 //
 // grog_gridding! (src/GROG.jl:73-102): per sample and dimension the grid index
 // follows the reference's float32/float64 promotion bit for bit, and
@@ -28,7 +29,10 @@
 namespace mrsr {
 
 constexpr int kGrogMaxCoils = 32;
-constexpr int kLogGL = 12;  // Gauss-Legendre nodes of the log quadrature
+// log(Y) = 2 atanh(Z), Z = (Y - I)(Y + I)^{-1}: 21 terms of the series, in blocks of three.  With
+// ||Y - I|| <= 0.8, |z| <= 2/3 and what is left out is below 1e-9 of the result.
+constexpr float kLogMax2 = 0.64f;  // 0.8^2
+constexpr int kLogBlocks = 7;
 
 // ------------------------------------------------------- spoke Grams ---
 // A = D1^H D1, B = D1^H D2 for spoke `blockIdx.x`; one thread per (i, j).  The sums run on
@@ -106,9 +110,14 @@ __global__ void __launch_bounds__(1024, 2) k_grog_gram(GramArgs a) {
 }
 
 // ------------------------------------------ small dense linear algebra ---
-// All routines: one CTA, n <= 32, column-major n x n complex matrices in shared
-// memory, templated on the complex type (double2 for the least squares solve,
-// float2 for the logarithm).
+// One CTA of four warps per spoke, n <= 32.  Matrices sit in registers, a warp on every fourth
+// column and lane r on row r, so an elimination step is two shuffles and four multiply-adds per
+// column and one barrier; only the pivot column goes through shared memory.  Pivoting is
+// implicit: rows stay where they are, the pivot of step k is the largest entry of column k in a
+// row not used before, and the permutation is undone when the result is written.
+constexpr int kGjWarps = 4;
+constexpr int kGjThreads = 32 * kGjWarps;
+constexpr int kGjCols = kGrogMaxCoils / kGjWarps;  // columns of an n x n matrix per warp
 
 template <class C> struct Cx;
 template <> struct Cx<double2> {
@@ -122,246 +131,370 @@ template <> struct Cx<float2> {
   static __device__ __forceinline__ float2 mk(float x, float y) { return make_float2(x, y); }
 };
 template <class C> __device__ __forceinline__ C cx_zero() { return Cx<C>::mk(0, 0); }
-template <class C> __device__ __forceinline__ C cx_sub(C a, C b) { return Cx<C>::mk(a.x - b.x, a.y - b.y); }
 template <class C> __device__ __forceinline__ C cx_mul(C a, C b) {
   return Cx<C>::mk(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+template <class C> __device__ __forceinline__ C cx_sub(C a, C b) { return Cx<C>::mk(a.x - b.x, a.y - b.y); }
+// a - b c
+template <class C> __device__ __forceinline__ C cx_msub(C a, C b, C c) {
+  return Cx<C>::mk(a.x - b.x * c.x + b.y * c.y, a.y - b.x * c.y - b.y * c.x);
 }
 template <class C> __device__ __forceinline__ typename Cx<C>::R cx_abs2(C a) { return a.x * a.x + a.y * a.y; }
 template <class C> __device__ __forceinline__ C cx_shfl(C v, int src) {
   return Cx<C>::mk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
-// Pivot bookkeeping of one Gauss-Jordan step, double-buffered by step parity.
+// Lane of the largest v >= 0 among the lanes of `in` (at least one); the first of equals.
+__device__ __forceinline__ int lane_of_max(float v, bool in) {
+  const unsigned key = in ? __float_as_uint(v) + 1u : 0u;  // non-negative floats order like their bits
+  return __ffs(__ballot_sync(0xffffffffu, key == __reduce_max_sync(0xffffffffu, key))) - 1;
+}
+__device__ __forceinline__ int lane_of_max(double v, bool in) {
+  const unsigned hi = in ? (unsigned)__double2hiint(v) + 1u : 0u;
+  const bool top = hi == __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = top ? (unsigned)__double2loint(v) : 0u;
+  const unsigned best = __reduce_max_sync(0xffffffffu, lo);
+  return __ffs(__ballot_sync(0xffffffffu, top && lo == best)) - 1;
+}
+
+// Pivot record of one elimination step, double-buffered by step parity.
 template <class C> struct GjStep {
-  C f[2][kGrogMaxCoils];  // column k after the row swap: the elimination multipliers
-  C rinv[2];              // 1 / pivot
+  C f[2][kGrogMaxCoils];  // column k
+  C rinv[2];              // 1 / pivot, 0 if |pivot|^2 < kTiny
   int p[2];               // pivot row
-  int sing[2];            // |pivot|^2 < kTiny: basic solution with x_k = 0
 };
 
-// Warp-wide pivot choice for column k, lane r holding row r: the first row r >= k of
-// largest modulus (partial pivoting); writes the step record `b`.
+// Pivot of a column (lane r holding row r) among the rows outside `used`, first of the largest;
+// writes record b.
 template <class C>
-__device__ __forceinline__ void gj_pivot(C v, int k, int n, GjStep<C>& st, int b) {
-  using R = typename Cx<C>::R;
+__device__ __forceinline__ void gj_pivot(C v, unsigned used, int n, GjStep<C>& st, int b) {
   const int lane = threadIdx.x & 31;
-  R best = (lane >= k && lane < n) ? cx_abs2(v) : R(-1);
-  int idx = lane;
-  for (int o = 16; o > 0; o >>= 1) {
-    const R ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (ob > best || (ob == best && oi < idx)) {
-      best = ob;
-      idx = oi;
-    }
-  }
-  int p = __shfl_sync(0xffffffffu, idx, 0);
-  if (p < k || p >= n) p = k;  // non-finite column: keep the row order (indices stay in range)
-  const C vk = cx_shfl(v, k), vp = cx_shfl(v, p);
-  if (lane < n) st.f[b][lane] = lane == p ? vk : v;
+  const int p = lane_of_max(cx_abs2(v), lane < n && !((used >> lane) & 1u));
+  const C vp = cx_shfl(v, p);
+  st.f[b][lane] = v;
   if (lane == 0) {
-    const R d = cx_abs2(vp);
+    const typename Cx<C>::R d = cx_abs2(vp);
     const bool s = !(d >= Cx<C>::kTiny);
     st.p[b] = p;
-    st.sing[b] = s;
     st.rinv[b] = s ? cx_zero<C>() : Cx<C>::mk(vp.x / d, -vp.y / d);
   }
 }
 
-// Solve M X = R in place (R <- X, M destroyed), partial pivoting.  One warp per column of
-// [M | R], lane r holding row r.  At step k only the columns of M right of k and all of R
-// are updated (M's columns <= k are never read again), and the warp that updates column
-// k+1 of M also picks the pivot of step k+1, so a step costs one barrier.
+// One step's shared part: the lane's multiplier (0 in the pivot row, and all 0 for a singular
+// column, whose unknown comes out as 0), the rows used so far, and what the pivot row's lane keeps.
 template <class C>
-__device__ void gj_solve(C* M, C* R, int n, GjStep<C>& st) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (warp == 0) gj_pivot(lane < n ? M[lane] : cx_zero<C>(), 0, n, st, 0);
+struct GjLane {
+  unsigned used = 0;
+  int step = 0;            // the step that took this lane's row
+  C rinv = cx_zero<C>();   // 1 / its pivot
+  __device__ __forceinline__ C take(const GjStep<C>& st, int k, int& p) {
+    const int lane = threadIdx.x & 31, b = k & 1;
+    p = st.p[b];
+    const C ri = st.rinv[b];
+    const C g = cx_mul(st.f[b][lane], ri);
+    used |= 1u << p;
+    if (lane == p) {
+      step = k;
+      rinv = ri;
+      return cx_zero<C>();
+    }
+    return g;
+  }
+};
+
+// X = A^{-1} B for column-major n x n A, B in global memory; out(i, j, X_ij).  The pivot row goes
+// through shared memory (rows[warp]), where one lane per column scales it: float64 runs at 1/60
+// of the float32 rate, and every lane scaling the entry it gets by a shuffle doubles its work.
+template <class C, class Out>
+__device__ __forceinline__ void gj_solve(const C* A, const C* B, int n, GjStep<C>& st, C (*rows)[2 * kGjCols], Out&& out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  C v[2 * kGjCols];  // columns of A, then of B
+#pragma unroll
+  for (int q = 0; q < kGjCols; ++q) {
+    const int c = warp + kGjWarps * q;
+    const bool in = lane < n && c < n;
+    v[q] = in ? A[lane + n * c] : cx_zero<C>();
+    v[kGjCols + q] = in ? B[lane + n * c] : cx_zero<C>();
+  }
+  unsigned used = 0;
+  int mine = 0;  // the step that took this lane's row
+  if (warp == 0) gj_pivot(v[0], used, n, st, 0);
   __syncthreads();
   for (int k = 0; k < n; ++k) {
-    const int b = k & 1;
-    const int p = st.p[b];
-    const bool sing = st.sing[b] != 0;
-    const C rinv = st.rinv[b];
-    const C f = lane < n ? st.f[b][lane] : cx_zero<C>();
-    // new value of row `lane` of column c from its old value vr
-    auto update = [&](int c, C vr) -> C {
-      const C vk = cx_shfl(vr, k), vp = cx_shfl(vr, p);
-      const C own = lane == p ? vk : vr;  // row `lane` after the swap of rows k and p
-      if (sing) return lane == k ? (c < n ? vp : cx_zero<C>()) : own;
-      const C rk = cx_mul(vp, rinv);
-      return lane == k ? rk : cx_sub(own, cx_mul(f, rk));
-    };
-    auto column = [&](int c) -> C* { return c < n ? M + n * c : R + n * (c - n); };
-    int c = k + 1 + warp;
-    // two columns at a time, so the loads and shuffles of one overlap those of the other;
-    // the warp's first column is k + 1 only in the first pair (warp 0)
-    for (; c + nw < 2 * n; c += 2 * nw) {
-      C* col0 = column(c);
-      C* col1 = column(c + nw);
-      const C v0 = lane < n ? col0[lane] : cx_zero<C>();
-      const C v1 = lane < n ? col1[lane] : cx_zero<C>();
-      const C n0 = update(c, v0), n1 = update(c + nw, v1);
-      if (lane < n) {
-        col0[lane] = n0;
-        col1[lane] = n1;
-      }
-      if (c == k + 1 && c < n) gj_pivot(n0, k + 1, n, st, b ^ 1);
+    const int b = k & 1, p = st.p[b];
+    const C ri = st.rinv[b], f = st.f[b][lane];
+    const bool sing = ri.x == 0 && ri.y == 0;
+    used |= 1u << p;
+    if (lane == p) {
+      mine = k;
+#pragma unroll
+      for (int q = 0; q < 2 * kGjCols; ++q) rows[warp][q] = v[q];
     }
-    if (c < 2 * n) {
-      C* col = column(c);
-      const C nv = update(c, lane < n ? col[lane] : cx_zero<C>());
-      if (lane < n) col[lane] = nv;
-      if (c == k + 1 && c < n) gj_pivot(nv, k + 1, n, st, b ^ 1);
+    __syncwarp();
+    if (lane < 2 * kGjCols) rows[warp][lane] = cx_mul(rows[warp][lane], ri);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 2 * kGjCols; ++q) {
+      const int c = warp + kGjWarps * q;  // columns of A up to k are not read again
+      const bool of_b = q >= kGjCols;
+      if (of_b || (c > k && c < n)) {
+        const C rk = rows[warp][q];
+        if (lane != p) {
+          if (!sing) v[q] = cx_sub(v[q], cx_mul(f, rk));
+        } else if (!sing || of_b) {  // a singular column: its unknown is 0
+          v[q] = rk;
+        }
+        if (!of_b && c == k + 1) gj_pivot(v[q], used, n, st, b ^ 1);
+      }
     }
     __syncthreads();
   }
+#pragma unroll
+  for (int q = 0; q < kGjCols; ++q) {
+    const int c = warp + kGjWarps * q;
+    if (lane < n && c < n) out(mine, c, v[kGjCols + q]);
+  }
 }
 
-// dst = src^{-1}; src is preserved (copied to scratch first).
-template <class C>
-__device__ void mat_inv(C* dst, const C* src, C* scratch, int n, GjStep<C>& st) {
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    scratch[e] = src[e];
-    dst[e] = Cx<C>::mk((e % n) == (e / n) ? 1 : 0, 0);
+// dst = A^{-1} (shared memory, column-major n x n) for the matrix whose entry (i, j) is a(i, j),
+// in place in registers: a processed column turns into a column of the inverse.  AtStep: pivot
+// rows are scaled by 1 / pivot at their step (twice the instructions).
+template <bool AtStep, class C, class In>
+__device__ __forceinline__ void gj_invert(C* dst, int n, GjStep<C>& st, In&& a) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  C v[kGjCols];
+  int pc[kGjCols];
+#pragma unroll
+  for (int q = 0; q < kGjCols; ++q) {
+    const int c = warp + kGjWarps * q;
+    v[q] = lane < n && c < n ? a(lane, c) : cx_zero<C>();
+    pc[q] = 0;
+  }
+  GjLane<C> own;
+  if (warp == 0) gj_pivot(v[0], own.used, n, st, 0);
+  __syncthreads();
+  for (int k = 0; k < n; ++k) {
+    int p;
+    const C g = own.take(st, k, p);
+    if constexpr (AtStep) {
+      const C ri = st.rinv[k & 1], f = st.f[k & 1][lane];
+      const bool sing = ri.x == 0 && ri.y == 0;
+#pragma unroll
+      for (int q = 0; q < kGjCols; ++q) {
+        const C rk = cx_mul(cx_shfl(v[q], p), ri);
+        if (lane != p) {
+          if (!sing) v[q] = cx_sub(v[q], cx_mul(f, rk));
+        } else if (!sing || warp + kGjWarps * q < k) {
+          v[q] = rk;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < kGjCols; ++q) v[q] = cx_msub(v[q], g, cx_shfl(v[q], p));
+    }
+    if (warp == k % kGjWarps) {  // column k: what is left of the unit column of row p
+#pragma unroll
+      for (int q = 0; q < kGjCols; ++q)
+        if (q == k / kGjWarps) {
+          v[q] = lane != p ? Cx<C>::mk(-g.x, -g.y) : AtStep ? own.rinv : Cx<C>::mk(1, 0);
+          pc[q] = p;
+        }
+    }
+    if (k + 1 < n && warp == (k + 1) % kGjWarps) {
+#pragma unroll
+      for (int q = 0; q < kGjCols; ++q)
+        if (q == (k + 1) / kGjWarps) gj_pivot(v[q], own.used, n, st, (k & 1) ^ 1);
+    }
+    __syncthreads();
+  }
+  // row p_i, column k holds entry (i, p_k) of the inverse (times pivot i)
+#pragma unroll
+  for (int q = 0; q < kGjCols; ++q) {
+    const int c = warp + kGjWarps * q;
+    if (lane < n && c < n) dst[own.step + n * pc[q]] = AtStep ? v[q] : cx_mul(v[q], own.rinv);
   }
   __syncthreads();
-  gj_solve(scratch, dst, n, st);
+}
+
+// acc[q] += (A B)(lane, warp + 4 q) for column-major n x n matrices in shared memory
+__device__ __forceinline__ void mat_mul_acc(float2* acc, const float2* A, const float2* B, int n) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = lane < n ? lane : 0;
+  auto step = [&](float2 u, int q, float2 v) {
+    acc[q].x = fmaf(u.x, v.x, fmaf(-u.y, v.y, acc[q].x));
+    acc[q].y = fmaf(u.x, v.y, fmaf(u.y, v.x, acc[q].y));
+  };
+  int l = 0;
+  if ((n & 1) == 0) {  // two entries of B per 16-byte load
+    for (; l < n; l += 2) {
+      const float2 u0 = A[row + n * l], u1 = A[row + n * (l + 1)];
+#pragma unroll
+      for (int q = 0; q < kGjCols; ++q) {
+        const int c = warp + kGjWarps * q;
+        if (c < n) {
+          const float4 v = *reinterpret_cast<const float4*>(B + l + n * c);
+          step(u0, q, make_float2(v.x, v.y));
+          step(u1, q, make_float2(v.z, v.w));
+        }
+      }
+    }
+  }
+  for (; l < n; ++l) {
+    const float2 u = A[row + n * l];
+#pragma unroll
+    for (int q = 0; q < kGjCols; ++q) {
+      const int c = warp + kGjWarps * q;
+      if (c < n) step(u, q, B[l + n * c]);
+    }
+  }
 }
 
 // Block sum of a per-thread value (all threads receive it).
-template <class R>
-__device__ __forceinline__ R block_sum(R acc, R* red) {
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+__device__ __forceinline__ float block_sum(float acc, float* red) {
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  R s = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
+  float s = 0.f;
+  for (int w = 0; w < kGjWarps; ++w) s += red[w];
   __syncthreads();
   return s;
 }
 
-// || Y - I ||_F^2
-template <class C>
-__device__ typename Cx<C>::R dist_eye2(const C* Y, int n, typename Cx<C>::R* red) {
-  typename Cx<C>::R acc = 0;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    C v = Y[e];
-    if ((e % n) == (e / n)) v.x -= 1;
-    acc += cx_abs2(v);
-  }
-  return block_sum(acc, red);
+// Per spoke: G = X^T in float32, X = A^{-1} B in float64 (A is a Gram matrix: its condition
+// number is the square of the data's).
+__global__ void __launch_bounds__(kGjThreads) k_grog_solve(const double2* AB, int n, float2* G) {
+  __shared__ GjStep<double2> st;
+  __shared__ double2 rows[kGjWarps][2 * kGjCols];
+  const int64_t nn = n * n;
+  const double2* A = AB + (int64_t)blockIdx.x * 2 * nn;
+  float2* g = G + (int64_t)blockIdx.x * nn;
+  gj_solve(A, A + nn, n, st, rows, [&](int i, int j, double2 x) { g[j + n * i] = make_float2((float)x.x, (float)x.y); });
 }
 
 struct LogArgs {
-  const double2* AB;    // [spoke][2][nc][nc]
+  const float2* G;      // [spoke][nc][nc]
   int nc;
   double2* vth;         // [spoke][nc][nc] = log(G)
-  const double* gl_t;   // Gauss-Legendre nodes on [0, 1]
-  const double* gl_w;
   int* err;
 };
 
-// One spoke: X = A^{-1} B in float64 (A is a Gram matrix: its condition number is the
-// square of the data's), G = X^T, v = log(G) in float32 (the reference works in the data's
-// float32 throughout).  Shared memory: the float64 pair (A, B) occupies the first 2 n^2
-// double2 slots, and the six float32 matrices alias them; G is written to the float slot
-// that overlaps A, which is dead once the solve ends.
-__global__ void __launch_bounds__(1024) k_grog_solve_log(LogArgs a) {
-  extern __shared__ __align__(16) unsigned char sraw[];
+// One spoke: v = log(G) in float32 (the reference works in the data's float32 throughout).
+// For 32 coils about 30 inversions and 40 products, bound by instruction issue: 1000 spokes take
+// 1.6 ms, and k_grog_solve 0.73 ms (float64 rate), against 5.9 ms for the two with the matrices
+// in shared memory, right-hand sides carried along and 12 inversions in the quadrature.
+__global__ void __launch_bounds__(kGjThreads, 7) k_grog_log(LogArgs a) {
+  extern __shared__ __align__(16) float2 lsm[];
   const int n = a.nc, nn = n * n;
-  __shared__ GjStep<double2> std_;
-  __shared__ GjStep<float2> stf;
-  __shared__ float red[32];
-  {
-    double2* Ad = reinterpret_cast<double2*>(sraw);
-    double2* Bd = Ad + nn;
-    const double2* AB = a.AB + (int64_t)blockIdx.x * 2 * nn;
-    for (int e = threadIdx.x; e < 2 * nn; e += blockDim.x) Ad[e] = AB[e];
-    __syncthreads();
-    gj_solve(Ad, Bd, n, std_);  // Bd = A^{-1} B = X
-    float2* Yf = reinterpret_cast<float2*>(sraw) + nn;  // second half of Ad
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-      const int i = e % n, j = e / n;
-      const double2 x = Bd[j + n * i];  // G = X^T
-      Yf[e] = make_float2((float)x.x, (float)x.y);
+  __shared__ GjStep<float2> st;
+  __shared__ float red[kGjWarps];
+  float2* Y = lsm;            // root iterate
+  float2* Z = lsm + nn;       // M of the iteration, then X
+  float2* T = lsm + 2 * nn;   // inverses
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // each thread owns the entries (lane, warp + 4 q) of every matrix
+  auto entries = [&](auto&& f) {
+#pragma unroll
+    for (int q = 0; q < kGjCols; ++q) {
+      const int c = warp + kGjWarps * q;
+      if (lane < n && c < n) f(q, lane + n * c, lane == c);
     }
-    __syncthreads();
-  }
-  float2* M = reinterpret_cast<float2*>(sraw);  // scratch
-  float2* Y = M + nn;                           // root iterate
-  float2* Z = M + 2 * nn;
-  float2* T1 = M + 3 * nn;
-  float2* T2 = M + 4 * nn;
-  float2* L = M + 5 * nn;                       // log accumulator
-  // inverse scaling: square roots until ||Y - I||_F <= 0.25, each by the product form of
+  };
+  const float2* G = a.G + (int64_t)blockIdx.x * nn;
+  entries([&](int, int e, bool) { Y[e] = G[e]; });
+  // inverse scaling: square roots until ||Y - I||_F <= 0.8, each by the product form of
   // the Denman-Beavers iteration (Cheng, Higham, Kenney and Laub, SIAM J. Matrix Anal.
   // Appl. 22, 2001): M0 = Y0 = A, Y <- Y (I + M^{-1}) / 2, M <- I/2 + (M + M^{-1}) / 4;
   // Y -> A^{1/2} and M -> I quadratically.  With Y = A^{1/2} (I + E), M = (I + E)^2 and the
   // step maps E to E^2 / 2: once ||M - I||_F^2 <= 1e-8 n, one more step brings E to the
-  // float32 rounding level.
+  // float32 rounding level.  Spokes have eigenvalues e^{i (pi - d)} with d down to 1e-4: the
+  // first root's M then comes within d^2 / 4 of singular, and what it gives depends on each
+  // rounding, so the inversions of the first two roots (and k_grog_solve) scale a pivot row at
+  // its step, the order the results of this code have always had; the following roots stay
+  // clear of the negative axis and their inversions scale the rows at the end.
   int s = 0;
-  while (s < 40 && dist_eye2(Y, n, red) > 0.0625f) {
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) Z[e] = Y[e];  // M
-    __syncthreads();
+  for (; s < 40; ++s) {
+    float d2 = 0.f;
+    entries([&](int, int e, bool diag) {
+      float2 v = Y[e];
+      Z[e] = v;
+      if (diag) v.x -= 1.f;
+      d2 += v.x * v.x + v.y * v.y;
+    });
+    if (!(block_sum(d2, red) > kLogMax2)) break;
     bool last = false;
     for (int it = 0; it < 40; ++it) {
-      mat_inv(T1, Z, M, n, stf);  // M^{-1}
-      for (int e = threadIdx.x; e < nn; e += blockDim.x) {  // T2 = Y (I + M^{-1})
-        const int i = e % n, j = e / n;
-        float2 acc = Y[i + n * j];
-        for (int l = 0; l < n; ++l) {
-          const float2 u = Y[i + n * l], v = T1[l + n * j];
-          acc.x = fmaf(u.x, v.x, fmaf(-u.y, v.y, acc.x));
-          acc.y = fmaf(u.x, v.y, fmaf(u.y, v.x, acc.y));
-        }
-        T2[e] = acc;
-      }
+      auto m = [&](int i, int j) { return Z[i + n * j]; };
+      if (s < 2)
+        gj_invert<true>(T, n, st, m);
+      else
+        gj_invert<false>(T, n, st, m);
+      float2 acc[kGjCols];
+      entries([&](int q, int e, bool) { acc[q] = Y[e]; });
+      mat_mul_acc(acc, Y, T, n);  // Y (I + M^{-1})
       __syncthreads();
       float dacc = 0.f;
-      for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-        const bool diag = (e % n) == (e / n);
-        Y[e] = make_float2(0.5f * T2[e].x, 0.5f * T2[e].y);
-        float2 m = make_float2(0.25f * (Z[e].x + T1[e].x) + (diag ? 0.5f : 0.f), 0.25f * (Z[e].y + T1[e].y));
+      entries([&](int q, int e, bool diag) {
+        Y[e] = make_float2(0.5f * acc[q].x, 0.5f * acc[q].y);
+        float2 m = make_float2(0.25f * (Z[e].x + T[e].x) + (diag ? 0.5f : 0.f), 0.25f * (Z[e].y + T[e].y));
         Z[e] = m;
         if (diag) m.x -= 1.f;
         dacc += m.x * m.x + m.y * m.y;
-      }
+      });
       const float tot = block_sum(dacc, red);
       if (last) break;
       last = tot <= 1e-8f * n;
     }
-    ++s;
   }
   if (s >= 40 && threadIdx.x == 0) atomicExch(a.err, 2);
-  // log(I + X), X = Y - I:  sum_j w_j X (I + t_j X)^{-1}
-  for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-    float2 v = Y[e];
-    if ((e % n) == (e / n)) v.x -= 1.f;
-    Z[e] = v;  // X
-    L[e] = make_float2(0.f, 0.f);
-  }
+  // 2 atanh(Z) = 2 Z sum_k W^k / (2 k + 1), W = Z^2, the sum by Horner's rule in W^3
+  gj_invert<false>(T, n, st, [&](int i, int j) {
+    const float2 v = Y[i + n * j];
+    return make_float2(v.x + (i == j ? 1.f : 0.f), v.y);
+  });
+  entries([&](int, int e, bool diag) {
+    if (diag) Y[e].x -= 1.f;
+  });
   __syncthreads();
-  for (int q = 0; q < kLogGL; ++q) {
-    const float tq = (float)a.gl_t[q], wq = (float)a.gl_w[q];
-    // solve (I + t X) W = X  ->  W = (I + t X)^{-1} X = X (I + t X)^{-1} (they commute)
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-      float2 v = make_float2(tq * Z[e].x, tq * Z[e].y);
-      if ((e % n) == (e / n)) v.x += 1.f;
-      M[e] = v;
-      T1[e] = Z[e];
+  float2 acc[kGjCols], w1[kGjCols], w2[kGjCols];
+  // acc = A B (+ what acc holds), stored to dst
+  auto product = [&](const float2* A, const float2* B, float2* dst, bool add) {
+    if (!add) {
+#pragma unroll
+      for (int q = 0; q < kGjCols; ++q) acc[q] = make_float2(0.f, 0.f);
     }
+    mat_mul_acc(acc, A, B, n);
     __syncthreads();
-    gj_solve(M, T1, n, stf);
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-      L[e].x = fmaf(wq, T1[e].x, L[e].x);
-      L[e].y = fmaf(wq, T1[e].y, L[e].y);
+    entries([&](int q, int e, bool) { dst[e] = acc[q]; });
+    __syncthreads();
+  };
+  product(Y, T, Z, false);  // Z
+  product(Z, Z, Y, false);  // W
+#pragma unroll
+  for (int q = 0; q < kGjCols; ++q) w1[q] = acc[q];
+  product(Y, Y, T, false);  // W^2
+#pragma unroll
+  for (int q = 0; q < kGjCols; ++q) w2[q] = acc[q];
+  product(Y, T, T, false);  // W^3
+  for (int b = kLogBlocks - 1; b >= 0; --b) {
+    const float c0 = 1.f / (float)(6 * b + 1), c1 = 1.f / (float)(6 * b + 3), c2 = 1.f / (float)(6 * b + 5);
+    entries([&](int q, int, bool diag) {
+      acc[q] = make_float2(fmaf(c2, w2[q].x, fmaf(c1, w1[q].x, diag ? c0 : 0.f)), fmaf(c2, w2[q].y, c1 * w1[q].y));
+    });
+    if (b == kLogBlocks - 1) {
+      entries([&](int q, int e, bool) { Y[e] = acc[q]; });
+      __syncthreads();
+    } else {
+      product(T, Y, Y, true);
     }
-    __syncthreads();
   }
-  const double sc = ldexp(1.0, s);
+#pragma unroll
+  for (int q = 0; q < kGjCols; ++q) acc[q] = make_float2(0.f, 0.f);
+  mat_mul_acc(acc, Z, Y, n);
+  const double sc = ldexp(2.0, s);
   double2* out = a.vth + (int64_t)blockIdx.x * nn;
-  for (int e = threadIdx.x; e < nn; e += blockDim.x) out[e] = make_double2(sc * L[e].x, sc * L[e].y);
+  entries([&](int q, int e, bool) { out[e] = make_double2(sc * acc[q].x, sc * acc[q].y); });
 }
+
 // nm (nspk x d) and the d x d pseudo-inverse factor P = (nm^T nm)^{-1}; single CTA.
 struct NmArgs {
   const float* trj;   // (d, ns_pf, nt)
@@ -422,23 +555,37 @@ __global__ void k_grog_nm(NmArgs a) {
   }
 }
 
-// lnG[d, i, j] = sum_p (P nm^T)[d, p] v[p, i, j] over all spokes (all repetitions).
-__global__ void k_grog_lng(const double* nm, const double* Pinv, const double2* vth, int d, int nc, int64_t nspk0,
-                           int nrep, float2* lnG) {
-  const int nn = nc * nc;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nn; e += gridDim.x * blockDim.x) {
-    double2 acc[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-    for (int rep = 0; rep < nrep; ++rep)
-      for (int64_t ip = 0; ip < nspk0; ++ip) {
-        const double2 v = vth[(rep * nspk0 + ip) * nn + e];
-        for (int dd = 0; dd < d; ++dd) {
-          double c = 0.0;
-          for (int q = 0; q < d; ++q) c += Pinv[dd * d + q] * nm[ip * d + q];
-          acc[dd].x += c * v.x;
-          acc[dd].y += c * v.y;
-        }
+// lnG[d, i, j] = sum_p (P nm^T)[d, p] v[p, i, j] over all spokes (all repetitions).  A block
+// takes 32 entries, its 32 warps every 32nd spoke, in float64, joined in a fixed order: 76 us
+// for 1000 spokes of 32 coils against 810 us for a thread per entry over all spokes.
+__global__ void __launch_bounds__(1024) k_grog_lng(const double* nm, const double* Pinv, const double2* vth, int d, int nc,
+                                                   int64_t nspk0, int nrep, float2* lnG) {
+  __shared__ double2 part[32][33];
+  const int nn = nc * nc, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane;
+  double2 acc[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
+  for (int64_t p = warp; p < nspk0 * nrep; p += 32) {
+    const int64_t ip = p % nspk0;
+    const double2 v = e < nn ? vth[p * nn + e] : make_double2(0, 0);
+    for (int dd = 0; dd < d; ++dd) {
+      double c = 0.0;
+      for (int q = 0; q < d; ++q) c += Pinv[dd * d + q] * nm[ip * d + q];
+      acc[dd].x += c * v.x;
+      acc[dd].y += c * v.y;
+    }
+  }
+  for (int dd = 0; dd < d; ++dd) {
+    part[warp][lane] = acc[dd];
+    __syncthreads();
+    if (warp == 0 && e < nn) {
+      double2 t = make_double2(0, 0);
+      for (int w = 0; w < 32; ++w) {
+        t.x += part[w][lane].x;
+        t.y += part[w][lane].y;
       }
-    for (int dd = 0; dd < d; ++dd) lnG[dd + (int64_t)d * e] = make_float2((float)acc[dd].x, (float)acc[dd].y);
+      lnG[dd + (int64_t)d * e] = make_float2((float)t.x, (float)t.y);
+    }
+    __syncthreads();
   }
 }
 
@@ -512,68 +659,139 @@ struct GridArgs {
   float h, lnorm;         // table spacing, ||lnG_dd||_1 (max column sum)
 };
 
-// One pass per dimension, in the reference's order.  One warp per (sample, frame); lane i
-// owns coil i of every repetition.  The matrices sit in shared memory column-major:
-// L at [0, n^2), table j at [(j + 1) n^2, (j + 2) n^2).
-__global__ void __launch_bounds__(1024, 1) k_grog_grid(GridArgs a) {
-  extern __shared__ float2 Ls[];
+// One pass per dimension, in the reference's order.  A warp takes 32 samples: lane i first works
+// out sample i's grid index, shift and polynomial degree (float64 as in the reference, once per
+// sample and not once per lane: float64 is 1/60 of the float32 rate), then lane i owns coil i and
+// the samples go through in fours.  Row i of L stays in lane i's registers; a product reads the
+// four vectors from shared memory, two entries per 16-byte broadcast load.  NC: coils rounded up
+// to a multiple of 8.  Table j sits at j n^2 in shared memory, column-major.
+// 512k samples, 32 coils: 0.96 ms a dimension against 2.17 ms with a shuffle pair per vector
+// entry and every lane repeating the float64 index arithmetic; bound by the shared-memory pipe
+// (80%) and by instruction issue (69%).
+constexpr int kGridWarps = 16, kGridFly = 4;
+
+template <int NC>
+__global__ void __launch_bounds__(32 * kGridWarps, 1) k_grog_grid(GridArgs a) {
+  extern __shared__ __align__(16) float2 gsm[];
+  __shared__ __align__(16) float2 wbuf[kGridWarps][kGridFly][NC];
   const int n = a.nc, nn = n * n, ntab = 2 * a.J + 1;
-  for (int e = threadIdx.x; e < nn; e += blockDim.x) Ls[e] = a.lnG[a.dd + (int64_t)a.d * e];
-  for (int e = threadIdx.x; e < ntab * nn; e += blockDim.x) Ls[nn + e] = a.tab[e];
+  for (int e = threadIdx.x; e < ntab * nn; e += blockDim.x) gsm[e] = a.tab[e];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool row = lane < n;
+  float2 Lr[NC];  // row `lane` of L
+#pragma unroll
+  for (int j = 0; j < NC; ++j) Lr[j] = row && j < n ? a.lnG[a.dd + (int64_t)a.d * (lane + n * j)] : make_float2(0.f, 0.f);
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t total = a.ns_pf * a.nt;
-  // y = M w for the n x n matrix M at `Mat` (lane i gets row i)
-  auto matvec = [&](const float2* Mat, float2 w) {
-    float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-    for (int j = 0; j < n; j += 2) {
-      const float2 w0 = make_float2(__shfl_sync(0xffffffffu, w.x, j), __shfl_sync(0xffffffffu, w.y, j));
-      const float2 w1 = make_float2(__shfl_sync(0xffffffffu, w.x, j + 1), __shfl_sync(0xffffffffu, w.y, j + 1));
-      if (lane < n) {
-        acc0 = cadd(acc0, cmul(Mat[lane + n * j], w0));
-        if (j + 1 < n) acc1 = cadd(acc1, cmul(Mat[lane + n * (j + 1)], w1));
-      }
-    }
-    return cadd(acc0, acc1);
+  const int64_t nwarps = (int64_t)gridDim.x * kGridWarps;
+  auto madd = [](float2& acc, float2 m, float x, float y) {
+    acc.x = fmaf(m.x, x, fmaf(-m.y, y, acc.x));
+    acc.y = fmaf(m.x, y, fmaf(m.y, x, acc.y));
   };
-  for (int64_t li = warp; li < total; li += nwarps) {
-    const float p = __fmul_rn(a.trj[a.dd + (int64_t)a.d * li], (float)a.Nd);  // Float32 * Int -> Float32
-    const double t = __dadd_rn((double)p, 0.5);                                // + 1/2 -> Float64
-    const double k = rint(t);                                                  // round: ties to even
-    const double shift = __ddiv_rn(__dmul_rn(__dsub_rn(k, t), (double)a.nr), (double)a.Nd);
-    if (lane == 0) a.trj_cart[a.dd + (int64_t)a.d * li] = (int32_t)((int64_t)k + a.Nd / 2);
-    const float s = (float)shift;
-    const int j = max(-a.J, min(a.J, (int)rintf(s / a.h)));
-    const float del = s - (float)j * a.h;
-    const float nrm = fabsf(del) * a.lnorm;
-    int q = 0;  // normally 0: the remainder is within half a table step
-    while (nrm > ldexpf(1.f, q) && q < 20) ++q;
-    const float x = ldexpf(nrm, -q), sq = ldexpf(del, -q);
-    int m = 0;  // smallest degree with x^(m+1) / (m+1)! <= 2^-27
-    for (float tm = x; tm > kGridTol && m < 30;) {
-      ++m;
-      tm *= x / (float)(m + 1);
-    }
-    const float2* Ej = Ls + (int64_t)(j + a.J + 1) * nn;
-    for (int rep = 0; rep < a.nrep; ++rep) {
-      float2 v = make_float2(0.f, 0.f);
-      const int64_t base = li + total * ((int64_t)a.nc * rep);
-      if (lane < n) v = a.data[base + total * lane];
-      for (int rr = 0; rr < (1 << q); ++rr) {
-        float2 w = v;  // Horner: w = v + (sq/m) L (v + (sq/(m-1)) L (... ))
-        for (int mm = m; mm >= 1; --mm) {
-          const float2 lw = matvec(Ls, w);
-          const float c = sq / (float)mm;
-          w = make_float2(v.x + c * lw.x, v.y + c * lw.y);
-        }
-        v = w;
+  for (int64_t l0 = ((int64_t)blockIdx.x * kGridWarps + w) * 32; l0 < total; l0 += nwarps * 32) {
+    // lane i: sample l0 + i
+    float del = 0.f;
+    int jt = 0, q = 0, m = 0;
+    if (l0 + lane < total) {
+      const int64_t li = l0 + lane;
+      const float p = __fmul_rn(a.trj[a.dd + (int64_t)a.d * li], (float)a.Nd);  // Float32 * Int -> Float32
+      const double t = __dadd_rn((double)p, 0.5);                                // + 1/2 -> Float64
+      const double k = rint(t);                                                  // round: ties to even
+      const double shift = __ddiv_rn(__dmul_rn(__dsub_rn(k, t), (double)a.nr), (double)a.Nd);
+      a.trj_cart[a.dd + (int64_t)a.d * li] = (int32_t)((int64_t)k + a.Nd / 2);
+      const float s = (float)shift;
+      jt = max(-a.J, min(a.J, (int)rintf(s / a.h)));
+      del = s - (float)jt * a.h;
+      const float nrm = fabsf(del) * a.lnorm;
+      while (nrm > ldexpf(1.f, q) && q < 20) ++q;  // normally 0: the remainder is within half a table step
+      const float x = ldexpf(nrm, -q);
+      del = ldexpf(del, -q);
+      for (float tm = x; tm > kGridTol && m < 30;) {  // smallest degree with x^(m+1) / (m+1)! <= 2^-27
+        ++m;
+        tm *= x / (float)(m + 1);
       }
-      v = matvec(Ej, v);
-      if (lane < n) a.data[base + total * lane] = v;
+    }
+    const int cnt = total - l0 < 32 ? (int)(total - l0) : 32;
+    for (int s0 = 0; s0 < cnt; s0 += kGridFly) {
+      float sq[kGridFly];
+      int js[kGridFly], reps[kGridFly], most = 1, deg = 0;
+#pragma unroll
+      for (int u = 0; u < kGridFly; ++u) {
+        sq[u] = __shfl_sync(0xffffffffu, del, s0 + u);
+        js[u] = __shfl_sync(0xffffffffu, jt, s0 + u) + a.J;
+        reps[u] = 1 << __shfl_sync(0xffffffffu, q, s0 + u);
+        most = max(most, reps[u]);
+        deg = max(deg, __shfl_sync(0xffffffffu, m, s0 + u));
+      }
+      for (int rep = 0; rep < a.nrep; ++rep) {
+        float2* base = a.data + l0 + s0 + total * ((int64_t)a.nc * rep + lane);
+        float2 v[kGridFly], z[kGridFly];
+#pragma unroll
+        for (int u = 0; u < kGridFly; ++u) v[u] = row && s0 + u < cnt ? base[u] : make_float2(0.f, 0.f);
+        for (int rr = 0; rr < most; ++rr) {
+#pragma unroll
+          for (int u = 0; u < kGridFly; ++u) z[u] = v[u];
+          for (int mm = deg; mm >= 1; --mm) {  // Horner: z = v + (sq/m) L (v + (sq/(m-1)) L (... ))
+            if (lane < NC) {
+#pragma unroll
+              for (int u = 0; u < kGridFly; ++u) wbuf[w][u][lane] = z[u];
+            }
+            __syncwarp();
+            float2 acc[kGridFly];
+#pragma unroll
+            for (int u = 0; u < kGridFly; ++u) acc[u] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < NC; j += 2) {
+#pragma unroll
+              for (int u = 0; u < kGridFly; ++u) {
+                const float4 x = *reinterpret_cast<const float4*>(&wbuf[w][u][j]);
+                madd(acc[u], Lr[j], x.x, x.y);
+                madd(acc[u], Lr[j + 1], x.z, x.w);
+              }
+            }
+            __syncwarp();
+            const float rm = 1.f / (float)mm;
+#pragma unroll
+            for (int u = 0; u < kGridFly; ++u) {
+              const float c = sq[u] * rm;
+              z[u] = make_float2(fmaf(c, acc[u].x, v[u].x), fmaf(c, acc[u].y, v[u].y));
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < kGridFly; ++u)
+            if (rr < reps[u]) v[u] = z[u];
+        }
+        // exp(s_j L) from the table
+        if (lane < NC) {
+#pragma unroll
+          for (int u = 0; u < kGridFly; ++u) wbuf[w][u][lane] = v[u];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kGridFly; ++u) {
+          const float2* E = gsm + js[u] * nn + (row ? lane : 0);
+          float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 8
+          for (int j = 0; j < n; ++j) {
+            const float2 x = wbuf[w][u][j];
+            madd(acc, E[n * j], x.x, x.y);
+          }
+          if (row && s0 + u < cnt) base[u] = acc;
+        }
+        __syncwarp();
+      }
     }
   }
+}
+
+template <int NC>
+static int launch_grog_grid(const GridArgs& g, int64_t total, int sms, cudaStream_t st) {
+  const size_t smem = sizeof(float2) * (size_t)(2 * g.J + 1) * g.nc * g.nc;
+  MRSR_CHECK_CUDA(cudaFuncSetAttribute(k_grog_grid<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(total, 32 * kGridWarps), sms));
+  k_grog_grid<NC><<<blocks, 32 * kGridWarps, smem, st>>>(g);
+  MRSR_LAUNCH_CHECK();
+  return MRSR_OK;
 }
 
 static int grog_sms() {
@@ -584,31 +802,6 @@ static int grog_sms() {
     return v > 0 ? v : 1;
   }();
   return n;
-}
-
-// Threads of the per-spoke logarithm CTA.
-constexpr unsigned kGrogLogThreads = 256;
-
-static void gauss_legendre01(int n, std::vector<double>& t, std::vector<double>& w) {
-  t.assign(n, 0.0);
-  w.assign(n, 0.0);
-  for (int i = 0; i < n; ++i) {
-    double z = std::cos(M_PI * (i + 0.75) / (n + 0.5)), pp = 0.0;
-    for (int it = 0; it < 100; ++it) {
-      double p1 = 1.0, p2 = 0.0;
-      for (int j = 1; j <= n; ++j) {
-        const double p3 = p2;
-        p2 = p1;
-        p1 = ((2.0 * j - 1.0) * z * p2 - (j - 1.0) * p3) / j;
-      }
-      pp = n * (z * p1 - p2) / (z * z - 1.0);
-      const double dz = p1 / pp;
-      z -= dz;
-      if (std::fabs(dz) < 1e-15) break;
-    }
-    t[i] = 0.5 * (1.0 - z);
-    w[i] = 1.0 / ((1.0 - z * z) * pp * pp);  // (2 / ((1-z^2) pp^2)) / 2 on [0, 1]
-  }
 }
 
 }  // namespace mrsr
@@ -628,33 +821,27 @@ extern "C" int mrsr_grog_calib(int ndims, int64_t nr, int64_t ns_per_frame, int6
   const int spf = (int)(ns_per_frame / nr);
   const int64_t nspk0 = (int64_t)spf * nt, nspk = nspk0 * nrep;
   const int nn = ncoils * ncoils;
-  DevBuf AB, vth, nm, Pinv, glt, glw, err;
+  DevBuf AB, G, vth, nm, Pinv, err;
   MRSR_TRY(AB.alloc(sizeof(double2) * 2 * nn * nspk));
+  MRSR_TRY(G.alloc(sizeof(float2) * nn * nspk));
   MRSR_TRY(vth.alloc(sizeof(double2) * nn * nspk));
   MRSR_TRY(nm.alloc(sizeof(double) * ndims * nspk0));
   MRSR_TRY(Pinv.alloc(sizeof(double) * 9));
-  std::vector<double> t, w;
-  gauss_legendre01(kLogGL, t, w);
-  MRSR_TRY(glt.alloc(sizeof(double) * kLogGL));
-  MRSR_TRY(glw.alloc(sizeof(double) * kLogGL));
-  MRSR_TRY(copy_h2d(glt.p, t.data(), sizeof(double) * kLogGL));
-  MRSR_TRY(copy_h2d(glw.p, w.data(), sizeof(double) * kLogGL));
   MRSR_TRY(err.alloc(sizeof(int)));
   MRSR_CHECK_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
   const size_t smem_g = sizeof(float2) * (kGramRows + 1) * (ncoils + 1);
   GramArgs ga{reinterpret_cast<const float2*>(data), ns_per_frame, nt, ncoils, nrep, (int)nr, spf, AB.as<double2>()};
   k_grog_gram<<<(unsigned)nspk, 1024, smem_g, st>>>(ga);
   MRSR_LAUNCH_CHECK();
-  const size_t smem_l = std::max(sizeof(double2) * 2, sizeof(float2) * 6) * nn;
-  // opt in whatever the size: the dynamic part plus the kernel's static pivot records can pass 48 KB
-  MRSR_CHECK_CUDA(cudaFuncSetAttribute(k_grog_solve_log, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_l));
-  LogArgs la{AB.as<double2>(), ncoils, vth.as<double2>(), glt.as<double>(), glw.as<double>(), err.as<int>()};
-  k_grog_solve_log<<<(unsigned)nspk, kGrogLogThreads, smem_l, st>>>(la);
+  k_grog_solve<<<(unsigned)nspk, kGjThreads, 0, st>>>(AB.as<double2>(), ncoils, G.as<float2>());
+  MRSR_LAUNCH_CHECK();
+  const LogArgs la{G.as<float2>(), ncoils, vth.as<double2>(), err.as<int>()};
+  k_grog_log<<<(unsigned)nspk, kGjThreads, sizeof(float2) * 3 * nn, st>>>(la);
   MRSR_LAUNCH_CHECK();
   NmArgs na{trj, ndims, (int)nr, spf, ns_per_frame, nt, nspk0, nm.as<double>(), Pinv.as<double>(), nrep};
   k_grog_nm<<<1, 1024, 0, st>>>(na);
   MRSR_LAUNCH_CHECK();
-  k_grog_lng<<<(unsigned)cdiv(nn, 128), 128, 0, st>>>(nm.as<double>(), Pinv.as<double>(), vth.as<double2>(), ndims,
+  k_grog_lng<<<(unsigned)cdiv(nn, 32), 1024, 0, st>>>(nm.as<double>(), Pinv.as<double>(), vth.as<double2>(), ndims,
                                                      ncoils, nspk0, nrep, reinterpret_cast<float2*>(lnG_out));
   MRSR_LAUNCH_CHECK();
   int herr = 0;
@@ -720,11 +907,12 @@ extern "C" int mrsr_grog_gridding(int ndims, const int64_t* img_shape, int64_t n
     g.nr = nr;
     g.h = hs;
     g.lnorm = lnorm;
-    const size_t smem = sizeof(float2) * (size_t)(2 * J + 2) * nn;
-    MRSR_CHECK_CUDA(cudaFuncSetAttribute(k_grog_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(total, 32), grog_sms()));
-    k_grog_grid<<<blocks, 1024, smem, st>>>(g);
-    MRSR_LAUNCH_CHECK();
+    switch ((ncoils + 7) / 8) {
+      case 1: MRSR_TRY(launch_grog_grid<8>(g, total, grog_sms(), st)); break;
+      case 2: MRSR_TRY(launch_grog_grid<16>(g, total, grog_sms(), st)); break;
+      case 3: MRSR_TRY(launch_grog_grid<24>(g, total, grog_sms(), st)); break;
+      default: MRSR_TRY(launch_grog_grid<32>(g, total, grog_sms(), st)); break;
+    }
   }
   MRSR_CHECK_CUDA(cudaStreamSynchronize(st));
   return MRSR_OK;
