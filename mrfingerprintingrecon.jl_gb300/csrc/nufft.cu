@@ -425,7 +425,7 @@ __device__ __forceinline__ void es_axis(float k, int M, float* w, int* idx) {
 
 // ------------------------------------------------------ tile sorts ---
 //
-// Samples counting-sorted by the tile (kTile or kSpTile cells a side, 2D and 3D) that holds
+// Samples counting-sorted by the tile (kTile3 or kSpTile cells a side) that holds
 // their first tap; a work item is a chunk of samples of one tile.  The samples are counted in
 // at most kSegs segments of consecutive ones, and a chunk takes whole segments of its tile, as
 // many as fit; a segment of a tile with more samples than a chunk takes is put in order first
@@ -434,9 +434,6 @@ __device__ __forceinline__ void es_axis(float k, int M, float* w, int* idx) {
 // does not depend on its chunk, takes one segment and no order.)
 constexpr int kSegs = 64;
 constexpr int kSegMin = 8192;               // samples per segment, at least
-constexpr int kTile = 12;                   // 2D interpolation windows
-constexpr int kWin = kTile + kEsWidth - 1;  // 19
-constexpr int kWinCells = kWin * kWin;      // 361
 constexpr int kChunk = 1024;                // samples per work item of the interpolation kernels
 constexpr int kTiledThreads = 512;
 
@@ -1121,12 +1118,12 @@ __global__ void k_bp_fold(BpFoldArgs a) {
 struct FwdPlaceArgs {
   int d;
   int64_t N[3], M[3], nimg, mcells;
-  int K, c;
+  int K, c;              // coil c + blockIdx.y
   Decomp dc;             // element -> (k, image position) over img x K
   const float2* x;       // (img..., K)
   const float2* cmaps;   // (img..., ncoils) or null
   const float* ipsi[3];
-  float2* g;             // [K][mcells], zeroed
+  float2* g;             // [coil][K][mcells], zeroed
 };
 
 __global__ void k_fwd_place(FwdPlaceArgs a) {
@@ -1144,8 +1141,8 @@ __global__ void k_fwd_place(FwdPlaceArgs a) {
       mul *= a.M[dd];
     }
     float2 v = a.x[e];
-    if (a.cmaps) v = cmul(a.cmaps[r + a.nimg * a.c], v);
-    a.g[(int64_t)k * a.mcells + l] = cscale(v, sc);
+    if (a.cmaps) v = cmul(a.cmaps[r + a.nimg * (a.c + (int)blockIdx.y)], v);
+    a.g[((int64_t)blockIdx.y * a.K + k) * a.mcells + l] = cscale(v, sc);
   }
 }
 
@@ -1231,90 +1228,108 @@ __global__ void __launch_bounds__(256) k_interp(InterpArgs a) {
   }
 }
 
-// 2D on the tile sort (the backprojection's 12 x 12 tiles and tap records): a work item,
-// up to 1024 samples whose first tap lies in one tile, loads the tile's 19 x 19-cell window of
-// the K interleaved planes into shared memory once, and each thread sums one sample's 64 taps
-// x K from the window.  Same weights and summation order as k_interp (w = (wy * 1) * wx,
-// taps y-major), so the data are bit-identical to it.
+// acc += (w, w) * g on both components at once
+__device__ __forceinline__ float2 fma2(float2 w, float2 g, float2 acc) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<const unsigned long long*>(&w)), "l"(*reinterpret_cast<const unsigned long long*>(&g)),
+        "l"(*reinterpret_cast<const unsigned long long*>(&acc)));
+  return *reinterpret_cast<float2*>(&r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<const unsigned long long*>(&a)), "l"(*reinterpret_cast<const unsigned long long*>(&b)));
+  return *reinterpret_cast<float2*>(&r);
+}
+
+// 2D on the tile sort (tiles of 16 x 16 cells): a work unit, up to 1024 samples of one tile and
+// a group of at most 16 planes (whole coils, K planes each), loads the group's 23 x 23-cell
+// window into shared memory ([cell][17], so that neither the loads along the cells nor the reads
+// along the planes meet a bank twice), and each half of a warp takes a sample, a lane per plane:
+// 64 taps of one 8-byte load and one packed multiply-add.  The lane of a coil's first plane then
+// sums the coil's planes times the basis.  All coils run in one launch.  Same weights and
+// summation order as k_interp (w = (wy * 1) * wx, taps y-major).
+// 256^2, 512k samples, 20 coils, K = 5: the whole forward model 1.50 against 4.14 ms, of which
+// this kernel took 3.3 ms with a thread per sample and one coil's K planes in the window (reads
+// at random cells meet banks twice and more); bound by the shared-memory reads (26 GB, 0.7 ms
+// at 128 bytes a cycle and SM).
+constexpr int kWinPitch = 17;
 struct InterpTiledArgs {
-  int M0, M1, K, c, u_complex, ntx;
-  int64_t nt, ns_tot;
+  int M0, M1, K, cpg, nc, c0, u_complex, ntx;
+  int64_t nt, ns_tot, cells;
   const void* U;
-  const float2* g;         // [mcells][K]
+  const float2* g;         // [nc * K][cells]
   float2* data;            // (ns_pf, nt, ncoils)
   const TapRec* rec;       // tap records in sorted order
   const int4* items;       // (tile, first sorted position, count, -)
   const int* nitems;
-  int* next;               // work counter, zeroed before the launch
+  unsigned long long* next;  // work counter, zeroed before the launch
 };
 
-__global__ void __launch_bounds__(kTiledThreads, 2) k_interp_tiled(InterpTiledArgs a) {
-  extern __shared__ float2 wk[];  // [kWinCells][K]
-  __shared__ int s_item;
-  const int K = a.K;
+__global__ void __launch_bounds__(kTiledThreads, 3) k_interp_tiled(InterpTiledArgs a) {
+  extern __shared__ float2 wk[];  // [kWinCells][kWinPitch]
+  __shared__ unsigned long long s_unit;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = kTiledThreads / 32;
+  const int half = lane >> 4, ch = lane & 15;
+  const int K = a.K, cl = ch / K, k0 = cl * K;  // the lane's coil in the group and its first plane
   const int nitems = *a.nitems;
+  const int ngroups = (a.nc + a.cpg - 1) / a.cpg;
+  const unsigned long long total = (unsigned long long)nitems * ngroups;
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(a.next, 1);
+    if (threadIdx.x == 0) s_unit = atomicAdd(a.next, 1ull);
     __syncthreads();
-    const int it = s_item;
-    if (it >= nitems) break;
-    const int4 item = a.items[it];
-    const int ox = (item.x % a.ntx) * kTile, oy = (item.x / a.ntx) * kTile;
-    for (int cw = threadIdx.x; cw < kWinCells; cw += blockDim.x) {
-      const int row = cw / kWin, col = cw - row * kWin;
-      const float2* src = a.g + (wrap32(ox + col, a.M0) + (int64_t)a.M0 * wrap32(oy + row, a.M1)) * K;
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (k < K) wk[cw * K + k] = src[k];
+    const unsigned long long u = s_unit;
+    if (u >= total) break;
+    const int grp = (int)(u / nitems);
+    const int4 item = a.items[u - (unsigned long long)grp * nitems];
+    const int ox = (item.x % a.ntx) * kSpTile, oy = (item.x / a.ntx) * kSpTile;
+    const int coils = min(a.cpg, a.nc - grp * a.cpg), np = coils * K;  // planes of the group
+    const float2* g = a.g + (int64_t)grp * a.cpg * K * a.cells;
+    for (int e = threadIdx.x; e < np * kWinCells; e += kTiledThreads) {
+      const int p = e / kWinCells, c = e - p * kWinCells;
+      const int row = c / kSpWin, col = c - row * kSpWin;
+      wk[c * kWinPitch + p] = g[p * a.cells + wrap32(ox + col, a.M0) + (int64_t)a.M0 * wrap32(oy + row, a.M1)];
     }
     __syncthreads();
-    for (int sidx = threadIdx.x; sidx < item.z; sidx += blockDim.x) {
-      const float4* r4 = reinterpret_cast<const float4*>(a.rec + item.y + sidx);
-      float wx[kEsWidth], wy[kEsWidth];
+    for (int s0 = warp * 2; s0 < item.z; s0 += nwarps * 2) {
+      const bool act = s0 + half < item.z;
+      const float4* r4 = reinterpret_cast<const float4*>(a.rec + item.y + (act ? s0 + half : s0));
+      float2 wx[kEsWidth];
+      float wy[kEsWidth];
       {
         const float4 q0 = r4[0], q1 = r4[1], q2 = r4[2], q3 = r4[3];
-        wx[0] = q0.x; wx[1] = q0.y; wx[2] = q0.z; wx[3] = q0.w;
-        wx[4] = q1.x; wx[5] = q1.y; wx[6] = q1.z; wx[7] = q1.w;
+        wx[0] = make_float2(q0.x, q0.x); wx[1] = make_float2(q0.y, q0.y);
+        wx[2] = make_float2(q0.z, q0.z); wx[3] = make_float2(q0.w, q0.w);
+        wx[4] = make_float2(q1.x, q1.x); wx[5] = make_float2(q1.y, q1.y);
+        wx[6] = make_float2(q1.z, q1.z); wx[7] = make_float2(q1.w, q1.w);
         wy[0] = q2.x; wy[1] = q2.y; wy[2] = q2.z; wy[3] = q2.w;
         wy[4] = q3.x; wy[5] = q3.y; wy[6] = q3.z; wy[7] = q3.w;
       }
       const int4 ri = reinterpret_cast<const int4*>(r4)[4];  // li, t, lx0, ly0
-      const int lx = ri.z - ox, ly = ri.w - oy;
-      float2 z[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) z[k] = make_float2(0.f, 0.f);
-      const bool in_win = (unsigned)lx < (unsigned)kTile && (unsigned)ly < (unsigned)kTile;
+      // the sort put the first tap in this tile (the same float arithmetic); the clamp keeps any
+      // other position inside the window
+      const int lx = min(max(ri.z - ox, 0), kSpTile - 1), ly = min(max(ri.w - oy, 0), kSpTile - 1);
+      const float2* w = wk + (ly * kSpWin + lx) * kWinPitch + (ch < np ? ch : 0);
+      float2 z = make_float2(0.f, 0.f);
 #pragma unroll
       for (int t2 = 0; t2 < kEsWidth; ++t2) {
-        const float w23 = wy[t2] * 1.f;
+        const float2 w23 = make_float2(wy[t2], wy[t2]);
 #pragma unroll
-        for (int t1 = 0; t1 < kEsWidth; ++t1) {
-          const float w = w23 * wx[t1];
-          // the sort put the first tap in this tile (the same float arithmetic); a sample
-          // outside it would read the grid itself
-          const float2* cell = in_win ? wk + ((ly + t2) * kWin + lx + t1) * K
-                                      : a.g + (wrap32(ri.z + t1, a.M0) + (int64_t)a.M0 * wrap32(ri.w + t2, a.M1)) * K;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (k < K) {
-              const float2 gv = cell[k];
-              z[k].x = fmaf(w, gv.x, z[k].x);
-              z[k].y = fmaf(w, gv.y, z[k].y);
-            }
-        }
+        for (int t1 = 0; t1 < kEsWidth; ++t1) z = fma2(mul2(w23, wx[t1]), w[(t2 * kSpWin + t1) * kWinPitch], z);
       }
-      const int64_t t = ri.y;
       float2 y = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (k < K) {
-          if (a.u_complex)
-            y = cadd(y, cmul(reinterpret_cast<const float2*>(a.U)[t + a.nt * k], z[k]));
-          else
-            y = cadd(y, cscale(z[k], reinterpret_cast<const float*>(a.U)[t + a.nt * k]));
-        }
+      for (int k = 0; k < K; ++k) {
+        const int src = (half << 4) | ((k0 + k) & 15);
+        const float2 zk = make_float2(__shfl_sync(0xffffffffu, z.x, src), __shfl_sync(0xffffffffu, z.y, src));
+        if (a.u_complex)
+          y = cadd(y, cmul(reinterpret_cast<const float2*>(a.U)[ri.y + a.nt * k], zk));
+        else
+          y = cadd(y, cscale(zk, reinterpret_cast<const float*>(a.U)[ri.y + a.nt * k]));
       }
-      a.data[ri.x + a.ns_tot * a.c] = y;
+      if (act && ch == k0 && cl < coils) a.data[ri.x + a.ns_tot * (a.c0 + grp * a.cpg + cl)] = y;
     }
     __syncthreads();
   }
@@ -1643,9 +1658,6 @@ extern "C" int mrsr_forward_model(int ndims, const int64_t* img_shape, int64_t n
   MRSR_TRY(fM.init(ndims, M));
   const float* ipsi[3] = {nullptr, nullptr, nullptr};
   for (int i = 0; i < ndims; ++i) MRSR_TRY(es_inv_psi_table(M[i], -(N[i] / 2), N[i], &ipsi[i]));
-  DevBuf grid, gridi;
-  MRSR_TRY(grid.alloc(sizeof(float2) * K * mcells));
-  MRSR_TRY(gridi.alloc(sizeof(float2) * K * mcells));
   // the interpolation runs on the tile sort of the samples (built once for all coils)
   TileSort ts;
   const bool small = sl.set.n < (1ll << 31) && ns_per_frame * nt < (1ll << 31);
@@ -1653,19 +1665,25 @@ extern "C" int mrsr_forward_model(int ndims, const int64_t* img_shape, int64_t n
   const int64_t ntiles3 = cdiv(M[0], kTile3) * cdiv(M[1], kTile3) * cdiv(M[2], kTile3);
   const bool tiled3 = ndims == 3 && small && ntiles3 < (1ll << 31) && mcells < (1ll << 32);
   if (tiled) {
-    MRSR_TRY(ts.build(sl.set, M, kTile, kChunk, false, st));
+    MRSR_TRY(ts.build(sl.set, M, kSpTile, kChunk, false, st));
     MRSR_TRY(ts.prep(sl.set, MRSR_DCF_NONE, nullptr, st));
   } else if (tiled3) {
     MRSR_TRY(ts.build(sl.set, M, kTile3, kChunk, false, st));
     MRSR_TRY(ts.prep(sl.set, MRSR_DCF_NONE, nullptr, st));
   }
-  const size_t win_bytes = sizeof(float2) * kWinCells * (size_t)K;
+  // coils per pass: all of a 2 GB batch in the 2D tile-sorted kernel, one elsewhere
+  const int cc = tiled ? (int)std::max<int64_t>(1, std::min<int64_t>(ncoils, (2ll << 30) / ((int64_t)sizeof(float2) * K * mcells))) : 1;
+  DevBuf grid, gridi;
+  MRSR_TRY(grid.alloc(sizeof(float2) * K * mcells * cc));
+  if (!tiled) MRSR_TRY(gridi.alloc(sizeof(float2) * K * mcells));
+  const size_t win_bytes = sizeof(float2) * kWinCells * kWinPitch;
   const size_t win3_bytes = sizeof(float2) * kWin3Cells * (size_t)K;
   if (tiled) MRSR_CHECK_CUDA(cudaFuncSetAttribute(k_interp_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)win_bytes));
   if (tiled3)
     MRSR_CHECK_CUDA(cudaFuncSetAttribute(k_interp_tiled3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)win3_bytes));
-  for (int c = 0; c < ncoils; ++c) {
-    MRSR_CHECK_CUDA(cudaMemsetAsync(grid.p, 0, sizeof(float2) * K * mcells, st));
+  for (int c = 0; c < ncoils; c += cc) {
+    const int nc = std::min(cc, ncoils - c);
+    MRSR_CHECK_CUDA(cudaMemsetAsync(grid.p, 0, sizeof(float2) * K * mcells * nc, st));
     FwdPlaceArgs pa;
     pa.d = ndims;
     for (int i = 0; i < 3; ++i) {
@@ -1681,11 +1699,13 @@ extern "C" int mrsr_forward_model(int ndims, const int64_t* img_shape, int64_t n
     pa.x = reinterpret_cast<const float2*>(x);
     pa.cmaps = reinterpret_cast<const float2*>(cmaps);
     pa.g = grid.as<float2>();
-    k_fwd_place<<<grid1d(nimg * K), 256, 0, st>>>(pa);
+    k_fwd_place<<<dim3(grid1d(nimg * K), nc), 256, 0, st>>>(pa);
     MRSR_LAUNCH_CHECK();
-    MRSR_TRY(fM.run(grid.as<float2>(), K, -1, 1.0f, st));
-    k_interleave<<<grid1d(mcells), 256, 0, st>>>(grid.as<float2>(), gridi.as<float2>(), K, mcells);
-    MRSR_LAUNCH_CHECK();
+    MRSR_TRY(fM.run(grid.as<float2>(), (int64_t)nc * K, -1, 1.0f, st));
+    if (!tiled) {
+      k_interleave<<<grid1d(mcells), 256, 0, st>>>(grid.as<float2>(), gridi.as<float2>(), K, mcells);
+      MRSR_LAUNCH_CHECK();
+    }
     InterpArgs ia{sl.set, {M[0], M[1], M[2]}, mcells, K, c, u_is_complex, U, gridi.as<float2>(),
                   reinterpret_cast<float2*>(data_out)};
     if (tiled3) {
@@ -1717,20 +1737,23 @@ extern "C" int mrsr_forward_model(int ndims, const int64_t* img_shape, int64_t n
       ta.M0 = (int)M[0];
       ta.M1 = (int)M[1];
       ta.K = K;
-      ta.c = c;
+      ta.cpg = 16 / K;
+      ta.nc = nc;
+      ta.c0 = c;
       ta.u_complex = u_is_complex;
       ta.ntx = ts.ntx;
       ta.nt = nt;
       ta.ns_tot = ns_per_frame * nt;
+      ta.cells = mcells;
       ta.U = U;
-      ta.g = gridi.as<float2>();
+      ta.g = grid.as<float2>();
       ta.data = reinterpret_cast<float2*>(data_out);
       ta.rec = ts.rec.as<TapRec>();
       ta.items = ts.items.as<int4>();
       ta.nitems = ts.nitems.as<int>();
-      ta.next = ts.next.as<int>();
-      MRSR_CHECK_CUDA(cudaMemsetAsync(ts.next.p, 0, sizeof(int), st));
-      k_interp_tiled<<<152 * 2, kTiledThreads, win_bytes, st>>>(ta);
+      ta.next = ts.next.as<unsigned long long>();
+      MRSR_CHECK_CUDA(cudaMemsetAsync(ts.next.p, 0, sizeof(unsigned long long), st));
+      k_interp_tiled<<<152 * 3, kTiledThreads, win_bytes, st>>>(ta);
     } else {
       k_interp<<<(unsigned)std::min<int64_t>(std::max<int64_t>(cdiv(sl.set.n, 256), 1), 152 * 64), 256, 0, st>>>(ia);
     }

@@ -36,6 +36,7 @@ namespace mrsr {
 
 constexpr int kSpTile = 16;
 constexpr int kSpWin = kSpTile + kEsWidth - 1;  // 23
+constexpr int kWinCells = kSpWin * kSpWin;
 constexpr int kSpWarps = 12;
 constexpr int kSpThreads = kSpWarps * 32;
 constexpr int kSpChunk = kSpThreads;          // samples of a chunk, at most: one per thread
