@@ -479,9 +479,10 @@ static RowTiling rows_tiling(int L, int lines_per_row, int64_t nrows, bool balan
 }
 
 // Columns per CTA of the middle passes: 16 are 128-byte rows (128^3, 16 coils: the apply 11.49 ->
-// 10.65 ms against 8 columns; 32, one line each a CTA, 10.94).
+// 10.65 ms against 8 columns; 32, one line each a CTA, 10.94); 8 for lines over 512 points, whose
+// two buffers of the generic kernel would not fit in shared memory at 16.
 static int mid_tc(const mrsr_normalop* op) {
-  int TC = 16;
+  int TC = op->geo.g[1] <= 512 ? 16 : 8;
   while (TC > 1 && op->geo.g[0] % TC) TC >>= 1;
   return TC;
 }
