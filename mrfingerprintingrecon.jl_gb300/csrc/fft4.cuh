@@ -26,7 +26,7 @@ __host__ __device__ constexpr int rdft_first_factor(int R) {
        : (R % 3 == 0 && R != 3) ? 3 : (R % 5 == 0 && R != 5) ? 5 : R;
 }
 __host__ __device__ constexpr int rdft_table_base(int R) {
-  return (32 % R == 0) ? 32 : (24 % R == 0) ? 24 : (20 % R == 0) ? 20 : (30 % R == 0) ? 30 : 0;
+  return (32 % R == 0) ? 32 : (24 % R == 0) ? 24 : (20 % R == 0) ? 20 : (30 % R == 0) ? 30 : (36 % R == 0) ? 36 : (25 % R == 0) ? 25 : 0;
 }
 
 // exp(S 2 pi i m / R) from the __constant__ tables (S = -1 forward, +1 inverse)
@@ -34,7 +34,7 @@ template <int R, int S>
 __device__ __forceinline__ float2 rtw(int m) {
   constexpr int B = rdft_table_base(R);
   static_assert(B != 0, "no twiddle table for this register DFT length");
-  const float2* t = (B == 32) ? c_tw32 : (B == 24) ? c_tw24 : (B == 20) ? c_tw20 : c_tw30;
+  const float2* t = (B == 32) ? c_tw32 : (B == 24) ? c_tw24 : (B == 20) ? c_tw20 : (B == 30) ? c_tw30 : (B == 36) ? c_tw36 : c_tw25;
   const float2 w = t[(m % R) * (B / R)];
   return make_float2(w.x, S * w.y);
 }

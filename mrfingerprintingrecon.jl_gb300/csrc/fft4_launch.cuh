@@ -2,21 +2,19 @@
 #pragma once
 #include "fft4.cuh"
 #include "passes.cuh"
+#include "splits.cuh"
 
 namespace mrsr {
 
 // -------------------------------------------------------- dispatch ---
 
+// the first group of lengths (the fp16-storage operator's)
 template <class F>
 inline int with_split(int L, F f) {
   switch (L) {
-    case 64: return f(Split<8, 8>());
-    case 128: return f(Split<8, 16>());
-    case 256: return f(Split<16, 16>());
-    case 384: return f(Split<12, 32>());
-    case 512: return f(Split<16, 32>());
-    case 768: return f(Split<24, 32>());
-    case 1024: return f(Split<32, 32>());
+#define MRSR_CASE(L_, R1_, R2_) case L_: return f(Split<R1_, R2_>());
+    MRSR_SPLITS_0(MRSR_CASE)
+#undef MRSR_CASE
     default: return MRSR_ERR_UNSUPPORTED;
   }
 }

@@ -11,6 +11,7 @@
 
 #include "fft4.cuh"
 #include "fftnd.cuh"
+#include "splits.cuh"
 
 namespace mrsr {
 
@@ -79,13 +80,9 @@ __global__ void __launch_bounds__(256) k_axis_fast(AxisArgs a, Slots sl) {
 template <class F>
 static int with_split_axis(int L, F f) {
   switch (L) {
-    case 64: return f(Split<8, 8>());
-    case 128: return f(Split<8, 16>());
-    case 256: return f(Split<16, 16>());
-    case 384: return f(Split<12, 32>());
-    case 512: return f(Split<16, 32>());
-    case 768: return f(Split<24, 32>());
-    case 1024: return f(Split<32, 32>());
+#define MRSR_CASE(L_, R1_, R2_) case L_: return f(Split<R1_, R2_>());
+    MRSR_SPLITS(MRSR_CASE)
+#undef MRSR_CASE
     default: return MRSR_ERR_UNSUPPORTED;
   }
 }
@@ -110,8 +107,7 @@ int fft_axis(float2* data, const FftPlan& pl, int64_t width, int64_t nouter, int
   a.sgn = (float)sign;
   a.scale = scale;
   a.data = data;
-  const bool fast = with_split_axis(L, [](auto) { return MRSR_OK; }) == MRSR_OK;
-  if (fast) {
+  if (split_length(L)) {
     return with_split_axis(L, [&](auto sp) -> int {
       using SP = decltype(sp);
       Slots sl;

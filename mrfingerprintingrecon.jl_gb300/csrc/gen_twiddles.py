@@ -8,7 +8,8 @@ from pathlib import Path
 
 import numpy as np
 
-BASES = (32, 24, 20, 30)
+BASES = (32, 24, 20, 30)  # fp16 register DFTs as well
+BASES32 = BASES + (36, 25)
 
 
 def half_bits(v):
@@ -18,7 +19,7 @@ def half_bits(v):
 def main():
     lines = ["// Generated by gen_twiddles.py: c_tw<R>[m] = (cos(2 pi m/R), sin(2 pi m/R)), m < R.",
              "#pragma once", "#include <cuda_runtime.h>", "", "namespace mrsr {", ""]
-    for R in BASES:
+    for R in BASES32:
         vals = []
         for m in range(R):
             a = 2.0 * math.pi * m / R

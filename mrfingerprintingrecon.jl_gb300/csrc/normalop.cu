@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "passes.cuh"
+#include "splits.cuh"
 
 namespace mrsr {
 
@@ -429,25 +430,13 @@ struct RowTiling {
 };
 
 
-// R1 of the register four-step split of L (apply_fast.cu's table), 0 if none
-static int fast_r1(int L) {
-  switch (L) {
-    case 64: case 128: return 8;
-    case 256: case 512: return 16;
-    case 384: return 12;
-    case 768: return 24;
-    case 1024: return 32;
-    default: return 0;
-  }
-}
-
 // Rows per CTA of the four-step forward row pass: the smallest count (up to twice the
 // line-element budget) whose step-B tasks rpc * lines * R1 best fill the CTA's threads
 // (a multiple of 32, at least 128, at most 256 per round).  For K = 5 lines of 512
 // points this is 2 rows (160 tasks, 160 threads) instead of 1 (80 tasks on 128 threads):
 // 0.043 -> 0.038 ms on 256^2 with 20 coils.
 static int balanced_rpc(int L, int lines, int64_t elems) {
-  const int r1 = fast_r1(L);
+  const int r1 = split_r1(L);
   const int rmax = (int)std::max<int64_t>(1, 2 * elems / ((int64_t)lines * L));
   int best = (int)std::max<int64_t>(1, elems / ((int64_t)lines * L));
   if (!r1) return best;
@@ -470,7 +459,7 @@ static RowTiling rows_tiling(int L, int lines_per_row, int64_t nrows, bool balan
   t.lstride = L;
   const int64_t elems = kRowElems;
   int rpc = (int)std::max<int64_t>(1, elems / ((int64_t)lines_per_row * L));
-  if (balance && fast_length(L)) rpc = balanced_rpc(L, lines_per_row, elems);
+  if (balance && split_length(L)) rpc = balanced_rpc(L, lines_per_row, elems);
   rpc = (int)std::min<int64_t>(rpc, nrows);
   t.rpc = rpc;
   t.threads = 256;
@@ -523,7 +512,7 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
       RowTiling t = rows_tiling(L1, Kr, nr, true);
       RowsFwdArgs a{op->plan[0].plan, (int)g.n[0], nr, t.rpc, Kr, c0, t.lstride, x, cm, st1};
       dim3 grid((unsigned)cdiv(nr, t.rpc), ncg);
-      if (fast_length(L1))
+      if (split_length(L1))
         MRSR_TRY(fast_rows_fwd(a, nr, ncg, st));
       else
         MRSR_TRY(launch_fft_kernel<RowsFwdArgs>(k_rows_fwd, grid, t.threads, t.smem, st, a));
@@ -539,7 +528,7 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
       MidArgs a{op->plan[1].plan, (int)g.n[1], L2, g.g[0], g.n[2], TC, NOo, L2 * TC, -1.f, st1, st2};
       dim3 grid((unsigned)(g.g[0] / TC), (unsigned)cdiv(g.n[2], NOo), (unsigned)(ncg * K));
       const size_t smem = sizeof(float2) * ((size_t)L2 + 2 * (size_t)NOo * a.lstride);
-      if (fast_length(L2))
+      if (split_length(L2))
         MRSR_TRY(fast_mid(a, ncg * K, st));
       else
         MRSR_TRY(launch_fft_kernel<MidArgs>(k_mid_fft, grid, 256, smem, st, a));
@@ -560,8 +549,8 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
         MRSR_TRY(tc_lambda(a, ncg, op->lam_max.as<float>(), op->tc_consts.p, op->errflag.as<int>(), st));
       } else if (lambda8_supported(a)) {
         MRSR_TRY(fast_lambda8(a, ncl, st));
-      } else if (fast_length(Ll))
-        MRSR_TRY(fast_lambda(a, ncl, op->Cg * K, op->errflag.as<int>(), st));
+      } else if (split_length(Ll))
+        MRSR_TRY(fast_lambda(a, ncl, st));
       else
         MRSR_TRY(launch_fft_kernel<LamPassArgs>(k_lambda_pass, grid, 512, smem, st, a));
       MRSR_TRY(rec.record());
@@ -574,7 +563,7 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
       MidArgs a{op->plan[1].plan, L2, (int)g.n[1], g.g[0], g.n[2], TC, NOo, L2 * TC, +1.f, st2, st1};
       dim3 grid((unsigned)(g.g[0] / TC), (unsigned)cdiv(g.n[2], NOo), (unsigned)(ncg * K));
       const size_t smem = sizeof(float2) * ((size_t)L2 + 2 * (size_t)NOo * a.lstride);
-      if (fast_length(L2))
+      if (split_length(L2))
         MRSR_TRY(fast_mid(a, ncg * K, st));
       else
         MRSR_TRY(launch_fft_kernel<MidArgs>(k_mid_fft, grid, 256, smem, st, a));
@@ -590,7 +579,7 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
         MRSR_TRY(tc_rows_inv(a, op->tc_consts.p, op->errflag.as<int>(), st));
       else if (rows8_inv_supported(a))
         MRSR_TRY(fast_rows8_inv(a, st));
-      else if (fast_length(L1))
+      else if (split_length(L1))
         MRSR_TRY(fast_rows_inv(a, nrows, st));
       else
         MRSR_TRY(launch_fft_kernel<RowsInvArgs>(k_rows_inv, grid, t.threads, t.smem, st, a));
@@ -644,7 +633,7 @@ int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_
   // Λ-pass tile width: up to 8 columns, a divisor of the plane width, <= 16384 elements per CTA
   // generic kernels: two K*TC*L buffers; four-step kernels: one K*TC*L exchange buffer (<= ~110 KB, 2 CTAs/SM)
   int TC = 8;
-  const int64_t budget = fast_length((int)g.glast()) ? 13000 : 12288;
+  const int64_t budget = split_length((int)g.glast()) ? 13000 : 12288;
   while (TC > 1 && ((int64_t)K * TC * g.glast() > budget || g.inner() % TC != 0)) TC >>= 1;
   op->TC = TC;
   if (precision == MRSR_PREC_FP16_TC) {

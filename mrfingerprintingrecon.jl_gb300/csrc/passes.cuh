@@ -158,11 +158,11 @@ __device__ __forceinline__ void lam_apply(const LamPassArgs& a, int64_t lbase, i
   lam_apply_ptr<KM>(a.lam_mode, a.K, a.lam, lbase, pstride, X, Y);
 }
 
-// Four-step fast paths (apply_fast.cu): return MRSR_ERR_UNSUPPORTED when the
-// transform length has no compiled split, so the caller uses the generic kernels.
+// Two-step fast paths (apply_fast.cuh, apply_lam.cuh): MRSR_ERR_UNSUPPORTED when the transform
+// length has no compiled split (splits.cuh); the caller uses the generic kernels there.
 bool fast_length(int L);
 int fast_rows_fwd(const RowsFwdArgs& a, int64_t nrows, int ncg, cudaStream_t st);
-int fast_lambda(const LamPassArgs& a, int ncg, int planes_total, int* errword, cudaStream_t st);
+int fast_lambda(const LamPassArgs& a, int ncg, cudaStream_t st);
 // three-step Λ pass (apply_lam8.cu): 256- or 512-point lines pruned to half, 4- or 8-column tiles, K <= 6
 bool lambda8_supported(const LamPassArgs& a);
 int fast_lambda8(const LamPassArgs& a, int ncg, cudaStream_t st);
