@@ -2,8 +2,7 @@
 //
 // Samples are counting-sorted by the tile (16 cells a side) that holds their first tap; the
 // footprints of a tile's samples lie in a window of 23 cells a side.  A work unit is a chunk
-// of at most 384 samples of one tile, in 3D one z-plane of the window, and up to 12 * 32 / P
-// rows of it; it takes the accumulator parts (the real and imaginary planes of the channels) in
+// of at most 384 samples of one tile and, in 3D, one z-plane of the window; it takes the accumulator parts (the real and imaginary planes of the channels) in
 // groups of P.  A lane owns one part of one window row and keeps the row's 23 sums in
 // registers, so a term costs one multiply-add and no shared-memory atomic.  The chunk's samples
 // are ordered by their x position in shared memory, and the loop over them is unrolled over the
@@ -175,9 +174,8 @@ __device__ __forceinline__ void sp_mad(unsigned long long& acc, unsigned v, unsi
 template <int P, int D, class Parts>
 __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a, Parts parts) {
   using Rec = typename std::conditional<D == 3, TapRec3, TapRec>::type;
-  constexpr int RW = 32 / P;                      // rows of a warp
-  constexpr int RU = kSpWarps * RW;               // rows of a unit
-  constexpr int NH = (kSpWin + RU - 1) / RU;      // row blocks of the window
+  constexpr int RW = 32 / P;                      // rows of a warp at a time
+  constexpr int RU = kSpWarps * RW;               // rows of the block at a time
   constexpr int NZ = D == 3 ? kSpWin : 1;         // window planes
   constexpr int NB = kSpChunk;
   constexpr int NK = kSpTile * kSpTile;           // (lx, ly) bins
@@ -195,22 +193,20 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
   const int part = lane % P, rsub = lane / P;
   const int nitems = *a.nitems;
   const int ngroups = (a.nparts + P - 1) / P;
-  const unsigned long long total = (unsigned long long)nitems * NZ * NH;
+  const unsigned long long total = (unsigned long long)nitems * NZ;
   const int e_grid = (int)((__float_as_uint(a.fs->scale) >> 23) & 255u) - 127 + kFxLoBits;
   const Rec* recs = reinterpret_cast<const Rec*>(a.rec);
   for (int b = tid; b < NK; b += kSpThreads) bins[b] = 0;
   for (;;) {
     if (tid == 0) s_unit = atomicAdd(a.next, 1ull);
     __syncthreads();
-    unsigned long long u = s_unit;
+    const unsigned long long u = s_unit;
     if (u >= total) break;
-    const int y0 = (int)(u % NH) * RU;
-    u /= NH;
     const int z = (int)(u % NZ);
     const int4 item = a.items[u / NZ];
     const int tx = item.x % a.ntx, tyz = item.x / a.ntx;
     const int ox = tx * kSpTile, oy = (D == 3 ? tyz % a.nty : tyz) * kSpTile, oz = (D == 3 ? tyz / a.nty : 0) * kSpTile;
-    // the samples whose footprint meets the unit's rows (and plane), counted by (lx, ly)
+    // the samples (in 3D, those whose footprint meets the plane), counted by (lx, ly)
     int key = -1, rank = 0;
     float4 ent = make_float4(0.f, 0.f, 0.f, 1.f);
     if (tid < item.z) {
@@ -218,7 +214,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
       const int4 ri = *reinterpret_cast<const int4*>(&r.li);  // li, t, lx0, ly0
       const int lx = ri.z - ox, ly = ri.w - oy;
       // the sort put the first tap in this tile (the same float arithmetic)
-      bool use = (unsigned)lx < (unsigned)kSpTile && (unsigned)ly < (unsigned)kSpTile && ly < y0 + RU && ly + kEsWidth > y0;
+      bool use = (unsigned)lx < (unsigned)kSpTile && (unsigned)ly < (unsigned)kSpTile;
       if constexpr (D == 3) {
         const int lz = r.lz0 - oz;
         use = use && (unsigned)lz < (unsigned)kSpTile && (unsigned)(z - lz) < (unsigned)kEsWidth;
@@ -289,9 +285,6 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
         }
       }
     }
-    // the warp's rows meet the samples of ly in [ylo, yhi)
-    const int wrow = y0 + warp * RW, row = wrow + rsub;
-    const int ylo = max(wrow - (kEsWidth - 1), 0), yhi = min(wrow + RW, kSpTile);
     for (int grp = 0; grp < ngroups; ++grp) {
       const int gpart = grp * P + part;
       const bool live = gpart < a.nparts;
@@ -321,8 +314,13 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
         }
       }
       __syncthreads();
-      // one x position at a time: which sums a sample meets is fixed in each of the unrolled loops
-      if (ylo < yhi) {
+      // The warp's rows, RU apart (a warp near the window's edge, whose rows few samples meet, has
+      // another one inside it), meet the samples of ly in [ylo, yhi), one x position at a time:
+      // which sums a sample meets is fixed in each of the unrolled loops.
+#pragma unroll 1
+      for (int wrow = warp * RW; wrow < kSpWin; wrow += RU) {
+        const int row = wrow + rsub;
+        const int ylo = max(wrow - (kEsWidth - 1), 0), yhi = min(wrow + RW, kSpTile);
         // acc 2^-(ea + 25) in units of 2^-e_grid: sh > 0, as the grid resolves 2^-40 of the
         // largest term and the products 2^-54 of the tile's
         const int sh = min(max(ea + kSpTapBits - e_grid, 1), 62);
