@@ -24,7 +24,9 @@ __global__ void __launch_bounds__(512) k4_rows_fwd(RowsFwdArgs a, Slots sl) {
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* sm = smem + L;
+  pdl_start();
   load_twiddles_a<SP>(tw, a.pl);
+  pdl_wait();
   const int cl = blockIdx.y;
   const int c = a.c0 + cl;
   const int64_t row0 = (int64_t)blockIdx.x * a.rpc;
@@ -57,7 +59,9 @@ __global__ void __launch_bounds__(512) k4_rows_inv(RowsInvArgs a, Slots sl) {
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* sm = smem + L;
+  pdl_start();
   load_twiddles_a<SP>(tw, a.pl);
+  pdl_wait();
   const int k = blockIdx.y;
   const int64_t row0 = (int64_t)blockIdx.x * a.rpc;
   const int nr = (int)min((int64_t)a.rpc, a.nrows - row0);
@@ -102,7 +106,9 @@ __global__ void __launch_bounds__(512) k4_mid(MidArgs a, Slots sl) {
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* sm = smem + L;
+  pdl_start();
   load_twiddles_a<SP>(tw, a.pl);
+  pdl_wait();
   const int64_t col0 = (int64_t)blockIdx.x * a.TC;
   const int64_t o0 = (int64_t)blockIdx.y * a.NOo;
   const int no = (int)min((int64_t)a.NOo, a.n3 - o0);

@@ -100,7 +100,9 @@ __global__ void __launch_bounds__(256, 2) k4_lambda(LamPassArgs a, SL sl) {
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* sm = smem + L;
+  pdl_start();
   load_twiddles(tw, a.pl);
+  pdl_wait();
   // coil fastest: the CTAs of one column tile run together and share its Λ tile in L2
   const int cl = (int)(blockIdx.x % (unsigned)a.ncg);
   const int64_t tile = blockIdx.x / (unsigned)a.ncg;

@@ -33,9 +33,7 @@ int launch(K k, dim3 grid, int threads, size_t smem, cudaStream_t st, const A& a
   MRSR_REQUIRE(smem <= 227 * 1024, MRSR_ERR_UNSUPPORTED, "shared memory request %zu too large", smem);
   if (smem > 48 * 1024) MRSR_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   MRSR_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  k<<<grid, threads, smem, st>>>(a, sl);
-  MRSR_LAUNCH_CHECK();
-  return MRSR_OK;
+  return launch_dependent(k, grid, threads, smem, st, a, sl);
 }
 
 }  // namespace mrsr

@@ -35,7 +35,9 @@ __global__ void __launch_bounds__(512) k_rows_fwd(RowsFwdArgs a) {
   float2* s = smem + a.pl.L;
   const int L = a.pl.L;
   float2* s1 = s + a.rpc * a.K * a.lstride;
+  pdl_start();
   load_twiddles(tw, a.pl);
+  pdl_wait();
   const int cl = blockIdx.y;
   const int c = a.c0 + cl;
   const int64_t row0 = (int64_t)blockIdx.x * a.rpc;
@@ -80,7 +82,9 @@ __global__ void __launch_bounds__(512) k_lambda_pass(LamPassArgs a) {
   float2* tw = smem;
   float2* s = smem + a.pl.L;
   float2* s1 = s + a.K * a.lstride;
+  pdl_start();
   load_twiddles(tw, a.pl);
+  pdl_wait();
   const int L = a.pl.L;
   const int cl = blockIdx.y;
   const int64_t tile = blockIdx.x;
@@ -145,7 +149,9 @@ __global__ void __launch_bounds__(512) k_mid_fft(MidArgs a) {
   float2* tw = smem;
   float2* s = smem + a.pl.L;
   float2* s1 = s + a.NOo * a.lstride;
+  pdl_start();
   load_twiddles(tw, a.pl);
+  pdl_wait();
   const int L = a.pl.L;
   const int64_t col0 = (int64_t)blockIdx.x * a.TC;
   const int64_t o0 = (int64_t)blockIdx.y * a.NOo;
@@ -190,7 +196,9 @@ __global__ void __launch_bounds__(512) k_rows_inv(RowsInvArgs a) {
   float2* tw = smem;
   float2* s = smem + a.pl.L;
   float2* s1 = s + a.rpc * a.ncg * a.lstride;
+  pdl_start();
   load_twiddles(tw, a.pl);
+  pdl_wait();
   const int L = a.pl.L;
   const int k = blockIdx.y;
   const int64_t row0 = (int64_t)blockIdx.x * a.rpc;
@@ -401,9 +409,7 @@ static int launch_fft_kernel(void (*k)(Args), dim3 grid, int threads, size_t sme
   MRSR_REQUIRE(smem <= 227 * 1024, MRSR_ERR_UNSUPPORTED, "shared memory request %zu too large", smem);
   if (smem > 48 * 1024) MRSR_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   MRSR_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  k<<<grid, threads, smem, st>>>(a);
-  MRSR_LAUNCH_CHECK();
-  return MRSR_OK;
+  return launch_dependent(k, grid, threads, smem, st, a);
 }
 
 struct Recorder {
