@@ -429,6 +429,7 @@ struct Recorder {
 // memory plus the twiddle table of the transform length.
 constexpr int64_t kRowElems = 4096;  // line elements per CTA of the row passes
 constexpr int64_t kMidElems = 4096;
+constexpr int kSms = 152;
 
 struct RowTiling {
   int threads, rpc, lstride;
@@ -460,13 +461,15 @@ static int balanced_rpc(int L, int lines, int64_t elems) {
   return best;
 }
 
-static RowTiling rows_tiling(int L, int lines_per_row, int64_t nrows, bool balance = false) {
+static RowTiling rows_tiling(int L, int lines_per_row, int64_t nrows, int others, bool balance = false) {
   RowTiling t;
   t.lstride = L;
   const int64_t elems = kRowElems;
   int rpc = (int)std::max<int64_t>(1, elems / ((int64_t)lines_per_row * L));
   if (balance && split_length(L)) rpc = balanced_rpc(L, lines_per_row, elems);
   rpc = (int)std::min<int64_t>(rpc, nrows);
+  // fewer rows where the CTAs (`others` of them per row block) would not reach every SM
+  while (rpc > 1 && cdiv(nrows, rpc) * others < kSms) rpc = (rpc + 1) / 2;
   t.rpc = rpc;
   t.threads = 256;
   t.smem = sizeof(float2) * ((size_t)L + 2 * (size_t)rpc * lines_per_row * t.lstride);
@@ -515,7 +518,7 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
     {
       const int Kr = flat_rows ? 1 : K;
       const int64_t nr = flat_rows ? nrows * K : nrows;
-      RowTiling t = rows_tiling(L1, Kr, nr, true);
+      RowTiling t = rows_tiling(L1, Kr, nr, ncg, true);
       RowsFwdArgs a{op->plan[0].plan, (int)g.n[0], nr, t.rpc, Kr, c0, t.lstride, x, cm, st1};
       dim3 grid((unsigned)cdiv(nr, t.rpc), ncg);
       if (split_length(L1))
@@ -577,7 +580,7 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
     }
     // P3: rows inverse + crop + coil combine
     {
-      RowTiling t = rows_tiling(L1, ncg, nrows);
+      RowTiling t = rows_tiling(L1, ncg, nrows, K);
       RowsInvArgs a{op->plan[0].plan, (int)g.n[0], nrows, t.rpc, K, c0, ncg, t.lstride, grp == 0 ? 1 : 0, al, beta,
                     st1, cm, y};
       dim3 grid((unsigned)cdiv(nrows, t.rpc), K);
@@ -641,6 +644,13 @@ int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_
   int TC = 8;
   const int64_t budget = split_length((int)g.glast()) ? 13000 : 12288;
   while (TC > 1 && ((int64_t)K * TC * g.glast() > budget || g.inner() % TC != 0)) TC >>= 1;
+  // narrower tiles where their CTAs (one per tile and coil, or per tile and plane of a stacked
+  // operator) would not reach every SM; 4 columns where the three-step pass takes the line
+  // (64^2, 4 coils, an apply alone 43.7 -> 38.5 us with the row passes' split below; 10
+  // iterations of CG on a few thousand pixels 10% faster)
+  const int64_t copies = kmax > KMAX ? K : ncoils;
+  const int tcmin = (g.glast() == 256 || g.glast() == 512) ? 4 : 2;
+  while (TC > tcmin && (g.inner() / TC) * copies < kSms) TC >>= 1;
   op->TC = TC;
   if (precision == MRSR_PREC_FP16_TC) {
     const int nl = (int)g.n[ndims - 1], gl = (int)g.glast();
