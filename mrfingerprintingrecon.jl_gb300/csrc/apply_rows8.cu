@@ -6,7 +6,7 @@
 // memory and its last sums the coils from registers: across the four lines of a group by
 // warp shuffles, across the groups in registers and, for the two thread halves, through
 // shared memory.  512-thread CTAs two per SM: 32 warps per SM against 16 for the two-step
-// kernel (apply_fast.cu), whose radix-32 register DFTs need 109 registers.  (The forward row
+// kernel (apply_fast.cuh), whose radix-32 register DFTs need 109 registers.  (The forward row
 // pass stays two-step: it writes twice what it reads and has one exchange instead of two, and
 // a three-step form measured 0.045 against 0.039 ms on 256^2 with 20 coils.)
 // src/NFFTNormalOp.jl:227-267 / ext/MRISubspaceReconCUDAExt/NFFTNormalOp.jl:193-218
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kL8Threads, 2) k8_rows_inv(RowsInvArgs a) {
   float2 acc[H];
 #pragma unroll
   for (int n1 = 0; n1 < H; ++n1) acc[n1] = make_float2(0.f, 0.f);
-  step_i3<C, G>(sm, o, [&](int i, const float2* v) {
+  step_i3<C, G>(sm, o, [&](const Round<C>&, int i, const float2* v) {
     const int cl = TC * (o.k1 + 2 * i) + o.li;
     if (cl >= a.ncg) return;
     if (a.cmaps) {

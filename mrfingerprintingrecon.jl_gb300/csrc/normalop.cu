@@ -651,6 +651,8 @@ int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_
   const int64_t copies = kmax > KMAX ? K : ncoils;
   const int tcmin = (g.glast() == 256 || g.glast() == 512) ? 4 : 2;
   while (TC > tcmin && (g.inner() / TC) * copies < kSms) TC >>= 1;
+  // two CTAs of the three-step pass per SM: 28 KB of a line tile per component at 8 columns
+  if (g.glast() == 384 && K * TC > 28) TC = std::min(TC, 4);
   op->TC = TC;
   if (precision == MRSR_PREC_FP16_TC) {
     const int nl = (int)g.n[ndims - 1], gl = (int)g.glast();
@@ -736,18 +738,15 @@ static LamLayout lam_layout(const mrsr_normalop* op) {
   return l;
 }
 
-// Λ chunk length: the largest divisor of L with at most 256 positions (FC*TC)
-// and at most 16 KB per chunk, so a chunk streams through a small shared ring.
+// Λ chunk length: the largest divisor of L with at most 256 positions (FC * TC), so the entries
+// of neighbouring frequencies and columns lie together.  The three-step pass wants all 256, also
+// where a chunk of a large kernel is over 16 KB (128^2, K = 6, 16 coils, an apply 63.9 -> 58.5 us;
+// 256^2 complex, K = 5, 20 coils 270 -> 221).
 static void choose_fc(mrsr_normalop* op) {
   const int L = (int)op->geo.glast();
-  const int esz = lam_is_real(op->lam_mode) ? 4 : 8;
   int best = 1;
-  for (int fc = 1; fc <= L; ++fc) {
-    if (L % fc) continue;
-    if ((int64_t)fc * op->TC > 256) continue;
-    if ((int64_t)fc * op->TC * op->P * esz > 16384) continue;
-    best = fc;
-  }
+  for (int fc = 1; fc <= L; ++fc)
+    if (L % fc == 0 && (int64_t)fc * op->TC <= 256) best = fc;
   op->FC = best;
 }
 
