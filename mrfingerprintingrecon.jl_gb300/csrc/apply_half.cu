@@ -1,7 +1,7 @@
 // Mixed-precision apply: the oversampled K-stack and the Toeplitz kernel are
 // stored in fp16 with one float32 scale per tile; all arithmetic (FFTs, the
 // K x K product, coil sums) is float32.  Same pass structure as the float32
-// four-step kernels (apply_fast.cu).  Each producing CTA writes its results to
+// two-step kernels (apply_fast.cuh).  Each producing CTA writes its results to
 // shared memory, reduces the largest component magnitude of its tile, and
 // stores value / scale as half2 with scale = max / kHalfTarget; the consumer
 // multiplies by the producer tile's scale when it loads.

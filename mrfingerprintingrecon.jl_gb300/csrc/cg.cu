@@ -87,6 +87,18 @@ __device__ __forceinline__ bool last_block(CgState* st, double2* partial, double
   return threadIdx.x == 0;
 }
 
+// body(i0, step) over a thread's elements i0, i0 + step, ... below n, kCgBatch at a time in that
+// order: a body loads all of its elements before it stores any, so their latencies overlap
+// (with a load and a store per element in turn, the stores held the next element's loads back;
+// 20 iterations on 192^2, K = 4, 12 coils 1727 -> 1690 us).
+constexpr int kCgBatch = 4;
+template <class F>
+__device__ __forceinline__ void for_batches(int64_t n, F&& body) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += kCgBatch * step)
+    body(i, step);
+}
+
 // x = 0, r = b, u = 0, res = |b|
 // Every vector kernel works on plane blockIdx.y of gridDim.y independent systems of n
 // unknowns each (one system for a plain solve), each with its own state and partials.
@@ -127,10 +139,18 @@ __global__ void k_cg_dir(const float2* r, float2* u, int64_t n, const CgState* s
   st += blockIdx.y;
   if (st->done) return;
   const float b = st->beta;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 rv = r[i], uv = u[i];
-    u[i] = make_float2(rv.x + b * uv.x, rv.y + b * uv.y);
-  }
+  for_batches(n, [&](int64_t i0, int64_t step) {
+    float2 rv[kCgBatch], uv[kCgBatch];
+#pragma unroll
+    for (int j = 0; j < kCgBatch; ++j)
+      if (i0 + j * step < n) {
+        rv[j] = r[i0 + j * step];
+        uv[j] = u[i0 + j * step];
+      }
+#pragma unroll
+    for (int j = 0; j < kCgBatch; ++j)
+      if (i0 + j * step < n) u[i0 + j * step] = make_float2(rv[j].x + b * uv[j].x, rv[j].y + b * uv[j].y);
+  });
 }
 
 // alpha = res^2 / <u, c>  (<u, c> = sum conj(u) c)
@@ -141,11 +161,21 @@ __global__ void k_cg_alpha(const float2* u, const float2* c, int64_t n, CgState*
   partial += (int64_t)blockIdx.y * gridDim.x;
   if (st->done) return;
   float re = 0.f, im = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 a = u[i], b = c[i];
-    re = fmaf(a.x, b.x, fmaf(a.y, b.y, re));
-    im = fmaf(a.x, b.y, fmaf(-a.y, b.x, im));
-  }
+  for_batches(n, [&](int64_t i0, int64_t step) {
+    float2 a[kCgBatch], b[kCgBatch];
+#pragma unroll
+    for (int j = 0; j < kCgBatch; ++j)
+      if (i0 + j * step < n) {
+        a[j] = u[i0 + j * step];
+        b[j] = c[i0 + j * step];
+      }
+#pragma unroll
+    for (int j = 0; j < kCgBatch; ++j)
+      if (i0 + j * step < n) {
+        re = fmaf(a[j].x, b[j].x, fmaf(a[j].y, b[j].y, re));
+        im = fmaf(a[j].x, b[j].y, fmaf(-a[j].y, b[j].x, im));
+      }
+  });
   double2 s = block_sum_f2(make_float2(re, im));
   double2 tot;
   if (last_block(st, partial, s, &tot)) {
@@ -169,17 +199,28 @@ __global__ void k_cg_update(float2* x, float2* r, const float2* u, const float2*
   if (st->done) return;
   const float ar = (float)st->ar, ai = (float)st->ai;
   float acc = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 uv = u[i], cv = c[i];
-    float2 xv = x[i], rv = r[i];
-    xv.x += ar * uv.x - ai * uv.y;
-    xv.y += ar * uv.y + ai * uv.x;
-    rv.x -= ar * cv.x - ai * cv.y;
-    rv.y -= ar * cv.y + ai * cv.x;
-    x[i] = xv;
-    r[i] = rv;
-    acc = fmaf(rv.x, rv.x, fmaf(rv.y, rv.y, acc));
-  }
+  for_batches(n, [&](int64_t i0, int64_t step) {
+    float2 uv[kCgBatch], cv[kCgBatch], xv[kCgBatch], rv[kCgBatch];
+#pragma unroll
+    for (int j = 0; j < kCgBatch; ++j)
+      if (i0 + j * step < n) {
+        uv[j] = u[i0 + j * step];
+        cv[j] = c[i0 + j * step];
+        xv[j] = x[i0 + j * step];
+        rv[j] = r[i0 + j * step];
+      }
+#pragma unroll
+    for (int j = 0; j < kCgBatch; ++j)
+      if (i0 + j * step < n) {
+        xv[j].x += ar * uv[j].x - ai * uv[j].y;
+        xv[j].y += ar * uv[j].y + ai * uv[j].x;
+        rv[j].x -= ar * cv[j].x - ai * cv[j].y;
+        rv[j].y -= ar * cv[j].y + ai * cv[j].x;
+        x[i0 + j * step] = xv[j];
+        r[i0 + j * step] = rv[j];
+        acc = fmaf(rv[j].x, rv[j].x, fmaf(rv[j].y, rv[j].y, acc));
+      }
+  });
   double2 s = block_sum_f2(make_float2(acc, 0.f));
   double2 tot;
   if (last_block(st, partial, s, &tot)) {

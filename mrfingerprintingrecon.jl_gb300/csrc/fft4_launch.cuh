@@ -1,4 +1,4 @@
-// Launch helpers of the register four-step kernels (apply_fast.cu, apply_lam.cu).
+// Launch helpers of the register two-step kernels (apply_fast.cuh, apply_lam.cuh).
 #pragma once
 #include "fft4.cuh"
 #include "passes.cuh"
