@@ -749,6 +749,7 @@ int TileSort::prep3(const SampleSet& S, int dcf_kind, const float* dcf, cudaStre
 }  // namespace mrsr
 
 #include "spread_rows.cuh"
+#include "spread_windows.cuh"
 
 namespace mrsr {
 
@@ -756,6 +757,7 @@ int spread_lambda(const SpreadLambdaArgs& a, const TileSort* ts, cudaStream_t st
   if (a.S.n == 0) return MRSR_OK;
   if (ts && ts->rec.p) {
     const LamParts parts{a.U, a.umax, a.u_complex, a.nq, a.p0, a.S.nt};
+    if (ts->tile != kSpTile) return spread_windows(a.M, a.cells, a.np * a.nq, a.q, a.fs, *ts, parts, st);
     return spread_rows(a.S.d, a.M, a.cells, a.np * a.nq, a.q, a.fs, *ts, parts, st);
   }
   MRSR_REQUIRE(a.cells < (1ll << 32), MRSR_ERR_UNSUPPORTED, "spreading grid of 2^32 cells or more");
@@ -770,6 +772,10 @@ int spread_lambda(const SpreadLambdaArgs& a, const TileSort* ts, cudaStream_t st
 
 int spread_data(const SpreadDataArgs& a, const TileSort* ts, cudaStream_t st) {
   if (a.S.n == 0) return MRSR_OK;
+  if (ts && a.U && ts->rec.p && ts->tile != kSpTile) {
+    const DataParts parts{a.data, a.U, nullptr, nullptr, a.u_complex, a.K, a.c0, a.nc, a.S.nt, a.S.ns_pf * a.S.nt};
+    return spread_windows(a.M, a.cells, 2 * a.nc * a.K, a.q, a.fs, *ts, parts, st);
+  }
   if (ts && a.U && ts->rec.p) {
     const unsigned gb = (unsigned)std::min<int64_t>(cdiv(a.S.n, 256), 152 * 16);
     MRSR_CHECK_CUDA(cudaMemsetAsync(a.tmax, 0, sizeof(float) * (size_t)ts->ntiles * a.nc, st));
@@ -996,15 +1002,16 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   MRSR_TRY(fG.init(d, G));
   const float* ipsi[3] = {nullptr, nullptr, nullptr};
   for (int i = 0; i < d; ++i) MRSR_TRY(es_inv_psi_table(M[i], -G[i] / 2, G[i] + 1, &ipsi[i]));
-  // channel batches of ~2 GB of upsampled float2 grid; the tile-sorted kernel takes at least
-  // eight parts per pass, so a 3D batch holds that many (8 GB each of float2 and fixed-point grid on 512^3)
+  // channel batches of ~2 GB of upsampled float2 grid; in 3D a batch fills the four parts of a
+  // window group
   const int nq = u_complex ? 2 : 1;  // a real basis spreads real values
   const int64_t max_bytes = 2ll << 30;
   int pb = (int)std::max<int64_t>(1, std::min<int64_t>(P, max_bytes / (mcells * (int64_t)sizeof(float2))));
-  if (d == 3) pb = std::max(pb, std::min(P, 8 / nq));
   const bool tiled = S.n < (1ll << 31) && S.ns_pf * S.nt < (1ll << 31);
+  const bool rows = tiled && (d == 2 || rows_pay(nq * pb, S.n, mcells));
+  if (d == 3 && !rows) pb = std::max(pb, std::min(P, kP3 / nq));
   DevBuf grid, qgrid, cgrid, fsb, umax;
-  const size_t qbytes = tiled ? spread_rows_bytes(nq * pb, mcells) : sizeof(long long) * nq * mcells * pb;
+  const size_t qbytes = rows ? spread_rows_bytes(nq * pb, mcells) : sizeof(long long) * nq * mcells * pb;
   MRSR_TRY(grid.alloc(sizeof(float2) * mcells * pb));
   MRSR_TRY(qgrid.alloc(qbytes));
   MRSR_TRY(cgrid.alloc(sizeof(float2) * gcells * P));
@@ -1020,9 +1027,9 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   }
   TileSort ts;
   const bool ordered = S.n < (1ll << 31) && d == 3;
-  if (tiled || ordered) MRSR_TRY(ts.build(S, M, kSpTile, kSpChunk, true, st));
-  if (tiled) {
-    MRSR_TRY(ts.prep(S, MRSR_DCF_NONE, nullptr, st));
+  if (tiled || ordered) MRSR_TRY(ts.build(S, M, rows ? kSpTile : kTile3, rows ? kSpChunk : kChunk, rows, st));
+  if (tiled) MRSR_TRY(ts.prep(S, MRSR_DCF_NONE, nullptr, st));
+  if (rows) {
     MRSR_TRY(umax.alloc(sizeof(float) * K));
     k_basis_max<<<K, 256, 0, st>>>(U, S.nt, u_complex, umax.as<float>());
     MRSR_LAUNCH_CHECK();
@@ -1032,11 +1039,11 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   // channels in batches of pb: spread, inverse DFT on the upsampled grid, deconvolve and fold onto the 2x grid
   for (int p0 = 0; p0 < P; p0 += pb) {
     const int np = std::min(pb, P - p0);
-    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, tiled ? spread_rows_bytes(nq * np, mcells) : sizeof(long long) * nq * mcells * np, st));
+    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, rows ? spread_rows_bytes(nq * np, mcells) : sizeof(long long) * nq * mcells * np, st));
     SpreadLambdaArgs sa{S, {M[0], M[1], M[2]}, mcells, U, u_complex, K, P, p0, np, nq, qgrid.as<long long>(),
                         fsb.as<FixedScale>(), umax.as<float>()};
     MRSR_TRY(spread_lambda(sa, tsp, st));
-    if (tiled)
+    if (rows)
       MRSR_TRY(parts_to_grid(qgrid.as<long long>(), nq, mcells, nq * np, fsb.as<FixedScale>(), grid.as<float2>(), st));
     else
       MRSR_TRY(fixed_to_grid(qgrid.as<long long>(), nq, mcells, np, fsb.as<FixedScale>(), grid.as<float2>(), st));
@@ -1553,10 +1560,11 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
   const bool tiled = U != nullptr && sl.set.n < (1ll << 31) && ns_per_frame * nt < (1ll << 31);
   const bool parts_layout = ndims == 3 && U != nullptr && !tiled && 2 * K <= 32;
   if (parts_layout) cc = std::min(cc, 16 / K);
+  const bool rows = tiled && (ndims == 2 || rows_pay(2 * K * cc, sl.set.n, mcells));
   DevBuf grid, qgrid, fsb;
   MRSR_TRY(grid.alloc((size_t)per_coil * cc));
   // fixed-point re and im, 8 bytes each
-  MRSR_TRY(qgrid.alloc(tiled ? spread_rows_bytes(2 * K * cc, mcells) : (size_t)per_coil * 2 * cc));
+  MRSR_TRY(qgrid.alloc(rows ? spread_rows_bytes(2 * K * cc, mcells) : (size_t)per_coil * 2 * cc));
   // fixed-point scale: |term component| <= max|data| max|U| (x2 for complex U) x dcf bound,
   // at most ceil(w / M) taps per sample, cell and dimension
   MRSR_TRY(fsb.alloc(sizeof(FixedScale)));
@@ -1584,9 +1592,9 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
   TileSort ts;
   DevBuf umax, tmax;
   const bool ordered = ndims == 3 && sl.set.n < (1ll << 31);
-  if (tiled || ordered) MRSR_TRY(ts.build(sl.set, M, kSpTile, kSpChunk, true, st));
-  if (tiled) {
-    MRSR_TRY(ts.prep(sl.set, dcf_kind, dcf_array, st));
+  if (tiled || ordered) MRSR_TRY(ts.build(sl.set, M, rows ? kSpTile : kTile3, rows ? kSpChunk : kChunk, rows, st));
+  if (tiled) MRSR_TRY(ts.prep(sl.set, dcf_kind, dcf_array, st));
+  if (rows) {
     MRSR_TRY(umax.alloc(sizeof(float) * K));
     MRSR_TRY(tmax.alloc(sizeof(float) * (size_t)ts.ntiles * cc));
     k_basis_max<<<K, 256, 0, st>>>(U, nt, u_is_complex, umax.as<float>());
@@ -1596,12 +1604,12 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
   if (cmaps) MRSR_CHECK_CUDA(cudaMemsetAsync(out, 0, sizeof(float2) * out_elems, st));
   for (int c0 = 0; c0 < ncoils; c0 += cc) {
     const int nc = std::min(cc, ncoils - c0);
-    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, tiled ? spread_rows_bytes(2 * K * nc, mcells) : (size_t)per_coil * 2 * nc, st));
+    MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, rows ? spread_rows_bytes(2 * K * nc, mcells) : (size_t)per_coil * 2 * nc, st));
     SpreadDataArgs sa{sl.set, {M[0], M[1], M[2]}, mcells, reinterpret_cast<const float2*>(data), c0, nc, U,
                       u_is_complex, K, dcf_kind, dcf_array, qgrid.as<long long>(), fsb.as<FixedScale>(), umax.as<float>(),
                       tmax.as<float>()};
     MRSR_TRY(spread_data(sa, tiled || ordered ? &ts : nullptr, st));
-    if (tiled) {
+    if (rows) {
       MRSR_TRY(parts_to_grid(qgrid.as<long long>(), 2, mcells, 2 * K * nc, fsb.as<FixedScale>(), grid.as<float2>(), st));
     } else if (parts_layout) {
       k_fixed_to_grid_cp<<<(unsigned)cdiv(mcells, 32), 256, 0, st>>>(qgrid.as<long long>(), 2 * nc * K, mcells,

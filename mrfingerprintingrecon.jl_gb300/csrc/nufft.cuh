@@ -100,6 +100,16 @@ __device__ __forceinline__ void fx_split(float a, int& hi, int& lo) {
   lo = __float_as_int(__fmaf_rn(d, (float)(1 << kFxLoBits), kMagic)) - kMagicBits;  // |lo| <= 2^20
 }
 
+// fx_split of the product a = x * y, the first rounding fused into the product
+__device__ __forceinline__ void fx_split_prod(float x, float y, int& hi, int& lo) {
+  constexpr float kMagic = 12582912.f;
+  constexpr int kMagicBits = 0x4B400000;
+  const float s1 = __fmaf_rn(x, y, kMagic);
+  hi = __float_as_int(s1) - kMagicBits;                          // round(x y)
+  const float d = __fmaf_rn(x, y, -__fsub_rn(s1, kMagic));       // x y - round(x y), |d| <= 1/2
+  lo = __float_as_int(__fmaf_rn(d, (float)(1 << kFxLoBits), kMagic)) - kMagicBits;
+}
+
 __device__ __forceinline__ long long fx_term(float a) {
   int hi, lo;
   fx_split(a, hi, lo);
@@ -126,7 +136,7 @@ struct SpreadLambdaArgs {
   int P;              // channels: packed pairs k1 <= k2
   int p0, np;         // spread only channels p0 .. p0+np-1
   int nq;             // parts per cell: 1 (real basis: the spread values are real) or 2
-  long long* q;       // [np][nq][cells], or the parts layout of spread_rows.cuh with tap records
+  long long* q;       // [np][nq][cells], or the parts layout of spread_rows.cuh on its tiles
   const FixedScale* fs;
   const float* umax;  // with tap records: k_basis_max of U
 };
@@ -158,7 +168,7 @@ struct SpreadDataArgs {
   int u_complex, K;
   int dcf_kind;
   const float* dcf;     // per kept sample (dcf_kind == array)
-  long long* q;         // [(c - c0) * K + k][2][cells], or the parts layout of spread_rows.cuh with tap records
+  long long* q;         // [(c - c0) * K + k][2][cells], or the parts layout of spread_rows.cuh on its tiles
   const FixedScale* fs;
   const float* umax;    // with tap records: k_basis_max of U, and room for ntiles * nc maxima
   float* tmax;

@@ -3,7 +3,7 @@
 // (486 and 648 would need 27 points), and 1024; R1 even, so that the zero-padded half of a line
 // is the first R1 / 2 inputs of a step-A task.  Other lengths run the generic shared-memory
 // kernels (fft.cuh), whose stages are divisions, barriers and two buffers (half the CTAs an SM):
-// 180 x 150, 12 coils, complex K = 3, an apply takes 152 us there and 55 us here.  In groups, one
+// 180 x 150, 12 coils, complex K = 3, an apply takes 152 us there and 48 us here.  In groups, one
 // translation unit per group and kernel family.
 #pragma once
 

@@ -1,8 +1,9 @@
 // Tile-sorted spreading with register accumulators (2D and 3D; nufft.cu).
 //
 // Samples are counting-sorted by the tile (16 cells a side) that holds their first tap; the
-// footprints of a tile's samples lie in a window of 23 cells a side.  A work unit is a chunk
-// of at most 384 samples of one tile and, in 3D, one z-plane of the window; it takes the accumulator parts (the real and imaginary planes of the channels) in
+// footprints of a tile's samples lie in a window of 23 cells a side.  A work unit is a chunk of at
+// most 384 samples of one tile and, in 3D, one z-plane of the window; it takes the window's rows
+// twelve at a time and the accumulator parts (the real and imaginary planes of the channels) in
 // groups of P.  A lane owns one part of one window row and keeps the row's 23 sums in
 // registers, so a term costs one multiply-add and no shared-memory atomic.  The chunk's samples
 // are ordered by their x position in shared memory, and the loop over them is unrolled over the
@@ -19,14 +20,14 @@
 // 64-bit sums as those of terms rounded to 2^-40 of the largest one (1.6e-7 on 256^2, 512k
 // samples, 20 coils; with 27 bits for the values instead of 29, 1.7e-7).
 //
-// 256^2, 512k samples, 20 coils, K = 5 (200 parts): 2.0 ms against 2.93 ms for windows of 32-bit
+// 256^2, 512k samples, 20 coils, K = 5 (200 parts): 1.51 ms against 2.93 ms for windows of 32-bit
 // limbs in shared memory, two shared atomics and about eight instructions per term; the 15
-// parts of the kernel precompute on 512^2: 0.25 against 0.46 ms; 64^3, 307k samples, 8 coils,
-// K = 4: 3.9 against 6.3 ms.  An inner step takes 20 instructions for the 8 terms of a sample
-// and row; it waits on shared-memory loads, and the stages around it (ordering, values, the
-// barriers of a 12-warp block at 24 warps per SM) take 40% of the time.  32 x 32 + 64-bit
-// multiply-adds alone run at 18 T/s, 32-bit shared atomics at 9.5 T/s, and a float form (two
-// limbs, four FMAs per term) at 7 T/s.
+// parts of the kernel precompute on 512^2: 0.23 against 0.46 ms; 64^3, 307k samples, 8 coils,
+// K = 4: 2.93 against 6.28 ms.  An inner step takes 20 instructions for the 8 terms of a sample
+// and row, at 24 warps per SM; it waits on shared-memory loads, and the stages around it
+// (ordering, values, barriers) take the rest of the time.  32 x 32 + 64-bit multiply-adds alone
+// run at 18 T/s, 32-bit shared atomics at 9.5 T/s, and a float form (two limbs, four FMAs per
+// term) at 7 T/s.
 // Tiles of 16: the flush is 2.07 (2D) or 2.97 (3D) atomics per grid cell and part, against
 // 2.5 and 6.6 with tiles of 12 (2D) and 8 (3D), and 64-bit atomics run at 0.73 T/s.
 #pragma once
@@ -74,7 +75,7 @@ struct LamParts {
     int k2 = 0;
     while ((k2 + 1) * (k2 + 2) / 2 <= p) ++k2;
     const int k1 = p - k2 * (k2 + 1) / 2;
-    return Lane{nt * k1, nt * k2, umax[k1] * umax[k2], q};
+    return Lane{nt * k1, nt * k2, umax ? umax[k1] * umax[k2] : 0.f, q};
   }
   __device__ __forceinline__ float value(const Lane& L, int, int t) const {
     if (u_complex) {
@@ -104,7 +105,7 @@ struct DataParts {
   };
   __device__ Lane bind(int part, int tile) const {
     const int ch = part >> 1, c = ch / K, k = ch - c * K;
-    return Lane{data + ns_tot * (c0 + c), nt * k, tmax[(int64_t)tile * nc + c] * umax[k], part & 1};
+    return Lane{data + ns_tot * (c0 + c), nt * k, tmax ? tmax[(int64_t)tile * nc + c] * umax[k] : 0.f, part & 1};
   }
   __device__ __forceinline__ float value(const Lane& L, int li, int t) const {
     if (u_complex) {
