@@ -460,6 +460,14 @@ static int parts_to_grid(const long long* q, int nq, int64_t cells, int nparts, 
   return MRSR_OK;
 }
 
+// Samples of a chunk: 384, fewer where 2D samples would not give every block a unit (a rule on the
+// number of samples alone, as chunks decide the rounding): 32^2, 12800 samples, 160 parts, a
+// backprojection 0.43 -> 0.27 ms, 8 parts 0.21 -> 0.19.
+inline int spread_chunk(int d, int64_t n) {
+  if (d == 3) return kSpChunk;
+  return (int)std::min<int64_t>(kSpChunk, std::max<int64_t>(64, cdiv(n, 304 * 32) * 32));
+}
+
 // bytes of the accumulators of `nparts` parts
 inline size_t spread_rows_bytes(int nparts, int64_t cells) {
   const int P = spread_lanes(nparts);
