@@ -1,4 +1,5 @@
-// Tile-sorted spreading with register accumulators (2D and 3D; nufft.cu).
+// Tile-sorted spreading with register accumulators (2D, and 3D where rows_pay in
+// spread_windows.cuh says so; nufft.cu).
 //
 // Samples are counting-sorted by the tile (16 cells a side) that holds their first tap; the
 // footprints of a tile's samples lie in a window of 23 cells a side.  A work unit is a chunk of at
