@@ -146,7 +146,8 @@ static int spread_windows(const int64_t* M, int64_t cells, int nparts, long long
 // parts 5.8 / 4.5, 15 parts 8.2 / 5.5; backprojection on 256^3 cells, 1.6M samples, 8 parts 5.5 /
 // 7.3, 16 parts 10.2 / 9.0, 32 parts 19.8 / 13.4; 4.9M samples, 24 parts 27.8 / 31.9, 32 parts
 // 36.7 / 32.2, 40 parts (48 lanes) 48.9 / 52.0; on 64^3 cells, 13k samples, 20 parts 0.42 / 0.48,
-// 32 parts 0.51 / 0.49.  Its padded grids cost memory: over 8 GiB a batch it is not taken (kernel precompute of 128^3, K = 5: 89 / 114 ms).
+// 32 parts 0.51 / 0.49.  Its padded grids cost memory: over 8 GiB a batch it is not taken (kernel
+// precompute of 128^3, K = 5: 89 / 114 ms).
 inline bool rows_pay(int parts, int total, int64_t n, int64_t cells) {
   auto padded = [](int p) { const int P = spread_lanes(p); return p ? cdiv(p, P) * P : 0; };
   const int64_t lanes = total / parts * padded(parts) + padded(total % parts);
