@@ -760,7 +760,7 @@ int spread_lambda(const SpreadLambdaArgs& a, const TileSort* ts, cudaStream_t st
   if (ts && ts->rec.p) {
     const LamParts parts{a.U, a.umax, a.u_complex, a.nq, a.p0, a.S.nt};
     if (ts->tile != kSpTile) return spread_windows(a.M, a.cells, a.np * a.nq, a.q, a.fs, *ts, parts, st);
-    return spread_rows(a.S.d, a.M, a.cells, a.np * a.nq, a.q, a.fs, *ts, parts, st);
+    return spread_rows(a.S.d, a.M, a.cells, a.np * a.nq, a.q, a.fs, a.bad, *ts, parts, st);
   }
   MRSR_REQUIRE(a.cells < (1ll << 32), MRSR_ERR_UNSUPPORTED, "spreading grid of 2^32 cells or more");
   const int* order = ts ? ts->order.as<int>() : nullptr;
@@ -785,7 +785,7 @@ int spread_data(const SpreadDataArgs& a, const TileSort* ts, cudaStream_t st) {
                                       reinterpret_cast<unsigned*>(a.tmax));
     MRSR_LAUNCH_CHECK();
     const DataParts parts{a.data, a.U, a.umax, a.tmax, a.u_complex, a.K, a.c0, a.nc, a.S.nt, a.S.ns_pf * a.S.nt};
-    return spread_rows(a.S.d, a.M, a.cells, 2 * a.nc * a.K, a.q, a.fs, *ts, parts, st);
+    return spread_rows(a.S.d, a.M, a.cells, 2 * a.nc * a.K, a.q, a.fs, a.bad, *ts, parts, st);
   }
   MRSR_REQUIRE(a.cells < (1ll << 32), MRSR_ERR_UNSUPPORTED, "spreading grid of 2^32 cells or more");
   const int* order = ts && a.S.d == 3 ? ts->order.as<int>() : nullptr;
@@ -804,11 +804,14 @@ int spread_data(const SpreadDataArgs& a, const TileSort* ts, cudaStream_t st) {
 
 // ------------------------------------------------------- fixed point ---
 
-// amax[slot] = max |f[i]| as float bits (non-negative floats order like their bit patterns)
-__global__ void k_absmax(const float* f, int64_t n, unsigned* amax) {
+// amax[slot] = max |f[i]| as float bits (non-negative floats order like their bit patterns), over the
+// finite entries with `finite`
+__global__ void k_absmax(const float* f, int64_t n, bool finite, unsigned* amax) {
   float m = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, fabsf(f[i]));
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float v = fabsf(f[i]);
+    if (!finite || finite_value(v)) m = fmaxf(m, v);
+  }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(amax, __float_as_uint(m));
 }
@@ -825,7 +828,7 @@ __global__ void k_fixed_scale(const unsigned* amax, int nf, double mult, double 
   out->inv = ldexpf(1.f, -e);
 }
 
-int fixed_scale(const float* const* f, const int64_t* n, int nf, double mult, double nterms, FixedScale* out,
+int fixed_scale(const float* const* f, const int64_t* n, int nf, double mult, double nterms, bool finite, FixedScale* out,
                 cudaStream_t st) {
   MRSR_REQUIRE(nf >= 0 && nf <= 3, MRSR_ERR_ARG, "fixed_scale: at most 3 factors");
   DevBuf am;
@@ -833,7 +836,7 @@ int fixed_scale(const float* const* f, const int64_t* n, int nf, double mult, do
   MRSR_CHECK_CUDA(cudaMemsetAsync(am.p, 0, 4 * sizeof(unsigned), st));
   for (int i = 0; i < nf; ++i) {
     const unsigned g = (unsigned)std::min<int64_t>(std::max<int64_t>(cdiv(n[i], 1024), 1), 152 * 8);
-    k_absmax<<<g, 256, 0, st>>>(f[i], n[i], am.as<unsigned>() + i);
+    k_absmax<<<g, 256, 0, st>>>(f[i], n[i], finite, am.as<unsigned>() + i);
     MRSR_LAUNCH_CHECK();
   }
   k_fixed_scale<<<1, 1, 0, st>>>(am.as<unsigned>(), nf, mult, nterms, out);
@@ -1012,7 +1015,7 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   const bool tiled = S.n < (1ll << 31) && S.ns_pf * S.nt < (1ll << 31);
   const bool rows = tiled && (d == 2 || rows_pay(nq * pb, nq * P, S.n, mcells));
   if (d == 3 && !rows) pb = std::max(pb, std::min(P, kP3 / nq));
-  DevBuf grid, qgrid, cgrid, fsb, umax;
+  DevBuf grid, qgrid, cgrid, fsb, umax, bad;
   const size_t qbytes = rows ? spread_rows_bytes(nq * pb, mcells) : sizeof(long long) * nq * mcells * pb;
   MRSR_TRY(grid.alloc(sizeof(float2) * mcells * pb));
   MRSR_TRY(qgrid.alloc(qbytes));
@@ -1025,7 +1028,7 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
     const int64_t nu = S.nt * (int64_t)K * (u_complex ? 2 : 1);
     const float* f[2] = {uf, uf};
     const int64_t n[2] = {nu, nu};
-    MRSR_TRY(fixed_scale(f, n, 2, u_complex ? 2.0 : 1.0, (double)S.n * taps_per_cell(d, M), fsb.as<FixedScale>(), st));
+    MRSR_TRY(fixed_scale(f, n, 2, u_complex ? 2.0 : 1.0, (double)S.n * taps_per_cell(d, M), rows, fsb.as<FixedScale>(), st));
   }
   TileSort ts;
   const bool ordered = S.n < (1ll << 31) && d == 3;
@@ -1033,6 +1036,7 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   if (tiled) MRSR_TRY(ts.prep(S, MRSR_DCF_NONE, nullptr, st));
   if (rows) {
     MRSR_TRY(umax.alloc(sizeof(float) * K));
+    MRSR_TRY(bad.alloc(sizeof(int) * nq * pb));
     k_basis_max<<<K, 256, 0, st>>>(U, S.nt, u_complex, umax.as<float>());
     MRSR_LAUNCH_CHECK();
   }
@@ -1043,10 +1047,11 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
     const int np = std::min(pb, P - p0);
     MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, rows ? spread_rows_bytes(nq * np, mcells) : sizeof(long long) * nq * mcells * np, st));
     SpreadLambdaArgs sa{S, {M[0], M[1], M[2]}, mcells, U, u_complex, K, P, p0, np, nq, qgrid.as<long long>(),
-                        fsb.as<FixedScale>(), umax.as<float>()};
+                        fsb.as<FixedScale>(), umax.as<float>(), bad.as<int>()};
     MRSR_TRY(spread_lambda(sa, tsp, st));
     if (rows)
-      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), nq, mcells, nq * np, fsb.as<FixedScale>(), grid.as<float2>(), st));
+      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), nq, mcells, nq * np, fsb.as<FixedScale>(), bad.as<int>(), grid.as<float2>(),
+                             st));
     else
       MRSR_TRY(fixed_to_grid(qgrid.as<long long>(), nq, mcells, np, fsb.as<FixedScale>(), grid.as<float2>(), st));
     MRSR_TRY(fM.run(grid.as<float2>(), np, +1, 1.0f, st));
@@ -1589,16 +1594,17 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
       f[nf] = dcf_array;
       n[nf++] = sl.set.n;
     }
-    MRSR_TRY(fixed_scale(f, n, nf, mult, (double)sl.set.n * taps_per_cell(ndims, M), fsb.as<FixedScale>(), st));
+    MRSR_TRY(fixed_scale(f, n, nf, mult, (double)sl.set.n * taps_per_cell(ndims, M), rows, fsb.as<FixedScale>(), st));
   }
   TileSort ts;
-  DevBuf umax, tmax;
+  DevBuf umax, tmax, bad;
   const bool ordered = ndims == 3 && sl.set.n < (1ll << 31);
   if (tiled || ordered) MRSR_TRY(ts.build(sl.set, M, rows ? kSpTile : kTile3, rows ? spread_chunk(ndims, sl.set.n) : kChunk, rows, st));
   if (tiled) MRSR_TRY(ts.prep(sl.set, dcf_kind, dcf_array, st));
   if (rows) {
     MRSR_TRY(umax.alloc(sizeof(float) * K));
     MRSR_TRY(tmax.alloc(sizeof(float) * (size_t)ts.ntiles * cc));
+    MRSR_TRY(bad.alloc(sizeof(int) * 2 * K * cc));
     k_basis_max<<<K, 256, 0, st>>>(U, nt, u_is_complex, umax.as<float>());
     MRSR_LAUNCH_CHECK();
   }
@@ -1609,10 +1615,11 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
     MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, rows ? spread_rows_bytes(2 * K * nc, mcells) : (size_t)per_coil * 2 * nc, st));
     SpreadDataArgs sa{sl.set, {M[0], M[1], M[2]}, mcells, reinterpret_cast<const float2*>(data), c0, nc, U,
                       u_is_complex, K, dcf_kind, dcf_array, qgrid.as<long long>(), fsb.as<FixedScale>(), umax.as<float>(),
-                      tmax.as<float>()};
+                      tmax.as<float>(), bad.as<int>()};
     MRSR_TRY(spread_data(sa, tiled || ordered ? &ts : nullptr, st));
     if (rows) {
-      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), 2, mcells, 2 * K * nc, fsb.as<FixedScale>(), grid.as<float2>(), st));
+      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), 2, mcells, 2 * K * nc, fsb.as<FixedScale>(), bad.as<int>(),
+                             grid.as<float2>(), st));
     } else if (parts_layout) {
       k_fixed_to_grid_cp<<<(unsigned)cdiv(mcells, 32), 256, 0, st>>>(qgrid.as<long long>(), 2 * nc * K, mcells,
                                                                     fsb.as<FixedScale>(), grid.as<float2>());

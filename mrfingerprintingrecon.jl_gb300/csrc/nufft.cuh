@@ -86,6 +86,9 @@ int es_inv_psi_table(int64_t M, int64_t jmin, int64_t count, const float** out);
 constexpr int kFxLoBits = 21;
 constexpr int kFxTermBits = 40;
 
+constexpr float kFltMax = 3.402823466e38f;
+__device__ __forceinline__ bool finite_value(float v) { return fabsf(v) <= kFltMax; }
+
 struct FixedScale {
   float scale;   // 2^(e - kFxLoBits): value * scale = a
   float inv;     // 2^-e
@@ -139,6 +142,7 @@ struct SpreadLambdaArgs {
   long long* q;       // [np][nq][cells], or the parts layout of spread_rows.cuh on its tiles
   const FixedScale* fs;
   const float* umax;  // with tap records: k_basis_max of U
+  int* bad;           // and room for a mark per part (spread_rows.cuh)
 };
 // Samples of a set counting-sorted by the tile (`tile` cells a side) of the grid M that holds
 // their first tap, in chunks (the work items of the tile-sorted kernels) of at most `most`
@@ -172,14 +176,15 @@ struct SpreadDataArgs {
   const FixedScale* fs;
   const float* umax;    // with tap records: k_basis_max of U, and room for ntiles * nc maxima
   float* tmax;
+  int* bad;             // and for a mark per part (spread_rows.cuh)
 };
 int spread_data(const SpreadDataArgs& a, const TileSort* ts, cudaStream_t st);
 
 // Scale of a fixed-point grid: every term's components are bounded by `mult` times the
 // product of the largest absolute entries of the nf (<= 3) factor arrays f[i] (n[i]
-// floats each), and a cell sums at most `nterms` terms.
-int fixed_scale(const float* const* f, const int64_t* n, int nf, double mult, double nterms, FixedScale* out,
-                cudaStream_t st);
+// floats each; with `finite`, of their finite entries), and a cell sums at most `nterms` terms.
+int fixed_scale(const float* const* f, const int64_t* n, int nf, double mult, double nterms, bool finite,
+                FixedScale* out, cudaStream_t st);
 
 // out[ch][cell] = complex(q[ch][0][cell], q[ch][1][cell] or 0) * 2^-e, for nch channels.
 int fixed_to_grid(const long long* q, int nq, int64_t cells, int64_t nch, const FixedScale* fs, float2* out,

@@ -21,6 +21,10 @@
 // 64-bit sums as those of terms rounded to 2^-40 of the largest one (1.6e-7 on 256^2, 512k
 // samples, 20 coils; with 27 bits for the values instead of 29, 1.7e-7).
 //
+// An integer cannot hold an infinity or a NaN, so a value that is not finite marks its part in
+// `bad`, and the conversion to float makes every cell of a marked part NaN, as a float sum's
+// transform would be.  The maxima run over finite entries, so the other parts are untouched.
+//
 // 256^2, 512k samples, 20 coils, K = 5 (200 parts): 1.51 ms against 2.93 ms for windows of 32-bit
 // limbs in shared memory, two shared atomics and about eight instructions per term; the 15
 // parts of the kernel precompute on 512^2: 0.23 against 0.46 ms; 64^3, 307k samples, 8 coils,
@@ -51,6 +55,7 @@ struct SpreadRowsArgs {
   int nparts;              // parts to spread
   long long* q;            // [ceil(nparts / P)][cells][P]
   const FixedScale* fs;
+  int* bad;                // [nparts], zeroed: set for parts that hold a value that is not finite
   int ntx, nty;
   const void* rec;         // TapRec (2D) or TapRec3 (3D) in sorted order
   const int4* items;       // (tile, first sorted position, count, -)
@@ -59,8 +64,8 @@ struct SpreadRowsArgs {
 };
 
 // Part p of the Λ precompute: pair p0 + p / nq (k1 <= k2, packed k2 (k2 + 1) / 2 + k1), plane
-// p % nq; value conj(U[t,k1]) U[t,k2] (k_spread_lambda's value).  umax[k]: largest |re| + |im|
-// of column k.
+// p % nq; value conj(U[t,k1]) U[t,k2] (k_spread_lambda's value).  umax[k]: largest finite
+// |re| + |im| of column k.
 struct LamParts {
   const void* U;
   const float* umax;
@@ -76,7 +81,7 @@ struct LamParts {
     int k2 = 0;
     while ((k2 + 1) * (k2 + 2) / 2 <= p) ++k2;
     const int k1 = p - k2 * (k2 + 1) / 2;
-    return Lane{nt * k1, nt * k2, umax ? umax[k1] * umax[k2] : 0.f, q};
+    return Lane{nt * k1, nt * k2, umax ? fminf(umax[k1] * umax[k2], kFltMax) : 0.f, q};
   }
   __device__ __forceinline__ float value(const Lane& L, int, int t) const {
     if (u_complex) {
@@ -91,7 +96,8 @@ struct LamParts {
 
 // Part p of the backprojection: channel p / 2 = (coil c0 + c) K + k, plane p % 2; value
 // y_c conj(U[t,k]) (k_spread_data's value; the tap weights carry the density compensation).
-// tmax[tile][c]: largest component of the tile's samples times their density compensation.
+// tmax[tile][c]: largest component of the tile's samples times their density compensation, infinite
+// if one of them is not finite (bd is NaN then).
 struct DataParts {
   const float2* data;
   const void* U;
@@ -106,7 +112,9 @@ struct DataParts {
   };
   __device__ Lane bind(int part, int tile) const {
     const int ch = part >> 1, c = ch / K, k = ch - c * K;
-    return Lane{data + ns_tot * (c0 + c), nt * k, tmax ? tmax[(int64_t)tile * nc + c] * umax[k] : 0.f, part & 1};
+    const float tm = tmax ? tmax[(int64_t)tile * nc + c] : 0.f;
+    const float bd = tmax ? fminf(tm * umax[k], kFltMax) : 0.f;
+    return Lane{data + ns_tot * (c0 + c), nt * k, finite_value(tm) ? bd : __int_as_float(0x7fc00000), part & 1};
   }
   __device__ __forceinline__ float value(const Lane& L, int li, int t) const {
     if (u_complex) {
@@ -118,7 +126,7 @@ struct DataParts {
   }
 };
 
-// umax[k] = max over t of |U[t,k]| (real) or |re| + |im| (complex); one block per column
+// umax[k] = max over t of |U[t,k]| (real) or |re| + |im| (complex) where finite; one block per column
 __global__ void k_basis_max(const void* U, int64_t nt, int cplx, float* umax) {
   __shared__ float red[32];
   const int k = blockIdx.x;
@@ -126,9 +134,11 @@ __global__ void k_basis_max(const void* U, int64_t nt, int cplx, float* umax) {
   for (int64_t t = threadIdx.x; t < nt; t += blockDim.x) {
     if (cplx) {
       const float2 u = reinterpret_cast<const float2*>(U)[t + nt * k];
-      m = fmaxf(m, fabsf(u.x) + fabsf(u.y));
+      const float v = fabsf(u.x) + fabsf(u.y);
+      if (finite_value(v)) m = fmaxf(m, v);
     } else {
-      m = fmaxf(m, fabsf(reinterpret_cast<const float*>(U)[t + nt * k]));
+      const float v = fabsf(reinterpret_cast<const float*>(U)[t + nt * k]);
+      if (finite_value(v)) m = fmaxf(m, v);
     }
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -141,8 +151,8 @@ __global__ void k_basis_max(const void* U, int64_t nt, int cplx, float* umax) {
 }
 
 // tmax[tile][c] (zeroed before) = largest max(|re|, |im|) * |density compensation| over the
-// tile's samples of coil c0 + c.  Neighbouring samples share a tile: one atomic per run of
-// equal tiles in a warp and coil.
+// tile's samples of coil c0 + c, infinite if one of them is not finite.  Neighbouring samples share
+// a tile: one atomic per run of equal tiles in a warp and coil.
 __global__ void k_tile_absmax(SampleSet S, const int* tile_of, const float2* data, int c0, int nc, int dcf_kind,
                               const float* dcf, unsigned* tmax) {
   const int64_t ns_tot = S.ns_pf * S.nt;
@@ -159,7 +169,8 @@ __global__ void k_tile_absmax(SampleSet S, const int* tile_of, const float2* dat
       unsigned b = 0;
       if (act) {
         const float2 y = data[li + ns_tot * (c0 + c)];
-        b = __float_as_uint(fmaxf(fabsf(y.x), fabsf(y.y)) * w);
+        const float v = fmaxf(fabsf(y.x), fabsf(y.y)) * w;
+        b = finite_value(y.x) && finite_value(y.y) && finite_value(v) ? __float_as_uint(v) : 0x7f800000u;
       }
       b = __reduce_max_sync(grp, b);
       if (lead && b) atomicMax(&tmax[(int64_t)tile * nc + c], b);
@@ -293,7 +304,8 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
       const typename Parts::Lane L = parts.bind(live ? gpart : 0, item.x);
       // 2^a: bound < 2^ex
       float bd = live ? L.bd : 0.f;
-      if (!(bd < __int_as_float(0x7f800000))) bd = 0.f;  // infinite or NaN input: no meaningful sum
+      bool bad = !(bd >= 0.f);
+      if (bad) bd = 0.f;
       const int ex = max((int)(__float_as_uint(bd) >> 23), 1) - 126;
       const int ea = min(kSpValBits - ex, 126);
       const float scale = bd > 0.f ? __int_as_float((ea + 127) << 23) : 0.f;
@@ -307,6 +319,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
           const float4 en = list[i];
           val[j] = live ? parts.value(L, __float_as_int(en.x), __float_as_int(en.y)) : 0.f;
           if constexpr (D == 3) val[j] *= en.w;
+          bad |= !finite_value(val[j]);
         }
 #pragma unroll
         for (int j = 0; j < 2 * kSpFly; ++j) {
@@ -315,6 +328,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
           slots[i * TW + part] = val[j] * scale;
         }
       }
+      if (bad) a.bad[gpart] = 1;
       __syncthreads();
       // The warp's rows, RU apart (a warp near the window's edge, whose rows few samples meet, has
       // another one inside it), meet the samples of ly in [ylo, yhi), one x position at a time:
@@ -411,12 +425,13 @@ static int launch_spread_rows(const SpreadRowsArgs& a, const Parts& parts, cudaS
 
 // q: [ceil(nparts / P)][cells][P] with P = spread_lanes(nparts), zeroed
 template <class Parts>
-static int spread_rows(int d, const int64_t* M, int64_t cells, int nparts, long long* q, const FixedScale* fs,
+static int spread_rows(int d, const int64_t* M, int64_t cells, int nparts, long long* q, const FixedScale* fs, int* bad,
                        const TileSort& ts, const Parts& parts, cudaStream_t st) {
   MRSR_REQUIRE(ts.tile == kSpTile && ts.m0 == (int)M[0] && ts.m1 == (int)M[1] && (d == 2 || ts.m2 == (int)M[2]),
                MRSR_ERR_STATE, "tile sort built for another grid");
   MRSR_REQUIRE(ts.rec.p != nullptr, MRSR_ERR_STATE, "tile sort without tap records");
-  const SpreadRowsArgs a{ts.m0, ts.m1, d == 3 ? ts.m2 : 1, cells, nparts, q, fs, ts.ntx, ts.nty, ts.rec.p,
+  MRSR_CHECK_CUDA(cudaMemsetAsync(bad, 0, sizeof(int) * nparts, st));
+  const SpreadRowsArgs a{ts.m0, ts.m1, d == 3 ? ts.m2 : 1, cells, nparts, q, fs, bad, ts.ntx, ts.nty, ts.rec.p,
                          ts.items.as<int4>(), ts.nitems.as<int>(), ts.next.as<unsigned long long>()};
   switch (spread_lanes(nparts)) {
     case 8: return d == 3 ? launch_spread_rows<8, 3>(a, parts, st) : launch_spread_rows<8, 2>(a, parts, st);
@@ -426,18 +441,24 @@ static int spread_rows(int d, const int64_t* M, int64_t cells, int nparts, long 
 }
 
 // [group][cell][P] accumulators -> out[channel][cell], channel = nq parts (re, and im or 0):
-// 64 cells of one group per block through a shared tile, coalesced on both sides.
+// 64 cells of one group per block through a shared tile, coalesced on both sides; NaN in the parts
+// that are marked in `bad`.
 template <int P>
 __global__ void __launch_bounds__(256) k_parts_to_grid(const long long* q, int nq, int64_t cells, int nparts,
-                                                       const FixedScale* fs, float2* out) {
+                                                       const FixedScale* fs, const int* bad, float2* out) {
   constexpr int NC = 64;
   __shared__ float tile[P][NC + 1];
-  const float inv = fs->inv;
+  __shared__ float inv[P];  // 2^-e, NaN for a marked part
   const int64_t cell0 = (int64_t)blockIdx.x * NC;
   const int grp = blockIdx.y;
   const int nc = cells - cell0 < NC ? (int)(cells - cell0) : NC;
   const long long* qg = q + ((int64_t)grp * cells + cell0) * P;
-  for (int e = threadIdx.x; e < nc * P; e += 256) tile[e % P][e / P] = fx_to_float(qg[e]) * inv;
+  if (threadIdx.x < P) {
+    const int p = grp * P + threadIdx.x;
+    inv[threadIdx.x] = p < nparts && bad[p] ? __int_as_float(0x7fc00000) : fs->inv;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < nc * P; e += 256) tile[e % P][e / P] = fx_to_float(qg[e]) * inv[e % P];
   __syncthreads();
   const int ncu = min(P, nparts - grp * P) / nq;  // channels of the group
   for (int e = threadIdx.x; e < ncu * NC; e += 256) {
@@ -447,16 +468,16 @@ __global__ void __launch_bounds__(256) k_parts_to_grid(const long long* q, int n
   }
 }
 
-static int parts_to_grid(const long long* q, int nq, int64_t cells, int nparts, const FixedScale* fs, float2* out,
-                         cudaStream_t st) {
+static int parts_to_grid(const long long* q, int nq, int64_t cells, int nparts, const FixedScale* fs, const int* bad,
+                         float2* out, cudaStream_t st) {
   const int P = spread_lanes(nparts);
   const dim3 g((unsigned)cdiv(cells, 64), (unsigned)cdiv(nparts, P));
   if (P == 8)
-    k_parts_to_grid<8><<<g, 256, 0, st>>>(q, nq, cells, nparts, fs, out);
+    k_parts_to_grid<8><<<g, 256, 0, st>>>(q, nq, cells, nparts, fs, bad, out);
   else if (P == 16)
-    k_parts_to_grid<16><<<g, 256, 0, st>>>(q, nq, cells, nparts, fs, out);
+    k_parts_to_grid<16><<<g, 256, 0, st>>>(q, nq, cells, nparts, fs, bad, out);
   else
-    k_parts_to_grid<32><<<g, 256, 0, st>>>(q, nq, cells, nparts, fs, out);
+    k_parts_to_grid<32><<<g, 256, 0, st>>>(q, nq, cells, nparts, fs, bad, out);
   MRSR_LAUNCH_CHECK();
   return MRSR_OK;
 }
