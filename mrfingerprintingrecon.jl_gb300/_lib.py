@@ -55,8 +55,9 @@ SIGNATURES = {
     "mrsr_cg_batch_launch": [p, p],
     "mrsr_cg_batch_result": [p, i32, C.POINTER(i32), C.POINTER(f64)],
     "mrsr_cg_batch_destroy": [p],
-    # internal test hook (include/mrsr_test.h), not part of the product ABI
+    # internal test hooks (include/mrsr_test.h), not part of the product ABI
     "mrsr_test_set_device_error": [p, i32, p],
+    "mrsr_test_lambda_pass": [p, C.POINTER(i32), C.POINTER(i32)],
 }
 _VOID = {"mrsr_normalop_destroy", "mrsr_cg_batch_destroy"}
 _STR = {"mrsr_last_error"}

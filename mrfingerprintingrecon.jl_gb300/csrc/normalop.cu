@@ -485,6 +485,20 @@ static int mid_tc(const mrsr_normalop* op) {
   return TC;
 }
 
+// the Λ pass on `stack`; a stacked operator's planes are so many coils of one plane
+static LamPassArgs lam_pass_args(const mrsr_normalop* op, float2* stack) {
+  const OpGeom& g = op->geo;
+  const int L = (int)g.glast(), n = (int)g.nlast();
+  return LamPassArgs{op->plan[g.ndims - 1].plan, n, n, n, g.inner(), op->TC, lam_is_diag(op->lam_mode) ? 1 : g.K,
+                     op->P, op->lam_mode, L * op->TC, op->lam.p, stack, op->FC, L / op->FC};
+}
+
+int lam_pass_steps(const mrsr_normalop* op) {
+  if (op->precision == MRSR_PREC_FP32 && lambda8_supported(lam_pass_args(op, op->geo.ndims == 3 ? op->stack2.as<float2>() : op->stack1.as<float2>())))
+    return 3;
+  return split_length((int)op->geo.glast()) ? 2 : 0;
+}
+
 static void record_cb(void* ctx) { static_cast<Recorder*>(ctx)->record(); }
 
 static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alpha, float2 beta, cudaStream_t st,
@@ -548,11 +562,10 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
     {
       const int Ll = (int)g.glast();
       const int TC = op->TC;
-      const int Kl = diag ? 1 : K, ncl = diag ? ncg * K : ncg;
-      LamPassArgs a{op->plan[g.ndims - 1].plan, (int)g.nlast(), (int)g.nlast(), (int)g.nlast(), g.inner(), TC, Kl,
-                    op->P, op->lam_mode, Ll * TC, op->lam.p, lam_stack, op->FC, (int)(Ll / op->FC)};
+      const int ncl = diag ? ncg * K : ncg;
+      LamPassArgs a = lam_pass_args(op, lam_stack);
       dim3 grid((unsigned)(g.inner() / TC), ncl);
-      const size_t smem = sizeof(float2) * ((size_t)Ll + 2 * (size_t)Kl * a.lstride);
+      const size_t smem = sizeof(float2) * ((size_t)Ll + 2 * (size_t)a.K * a.lstride);
       if (op->precision == MRSR_PREC_FP16_TC) {
         a.lam = op->lam_tc.p;
         MRSR_TRY(tc_lambda(a, ncg, op->lam_max.as<float>(), op->tc_consts.p, op->errflag.as<int>(), st));
@@ -612,6 +625,32 @@ int normalop_apply_internal(mrsr_normalop* op, const float2* x, float2* y, float
 
 // ---------------------------------------------------------- builders ---
 
+// Λ-pass tile width: up to 8 columns, a divisor of the plane width, <= 16384 elements per CTA
+// (generic kernels: two K*TC*L buffers; two-step kernels: one K*TC*L exchange buffer, <= ~110 KB,
+// two CTAs per SM), for the operator's coil count.
+static int lam_tile_width(const mrsr_normalop* op, bool stacked) {
+  const OpGeom& g = op->geo;
+  const int L = (int)g.glast();
+  int TC = 8;
+  const int64_t budget = split_length(L) ? 13000 : 12288;
+  while (TC > 1 && ((int64_t)g.K * TC * L > budget || g.inner() % TC != 0)) TC >>= 1;
+  int lo, hi;
+  const bool tiles = lambda8_tiles(L, &lo, &hi);
+  const bool three = tiles && op->kind == MRSR_KIND_NFFT && op->precision == MRSR_PREC_FP32 && !stacked && g.K <= kL8MaxK;
+  // the three-step pass: a compiled tile, narrow enough for two CTAs per SM (an apply of 384^2, 20
+  // coils, K = 1 159 us with 8 columns, two-step, 129 with 4; K = 4 complex 585 us with 4, 529 with
+  // 2; 256^2, 20 coils, K = 3 complex 159 us with 8, 137 with 4)
+  if (three) TC = std::min(TC, hi);
+  while (three && TC > lo && !lambda8_two_per_sm(L, TC, g.K)) TC >>= 1;
+  // narrower tiles where their CTAs (one per tile and coil, or per tile and plane of a stacked
+  // operator) would not reach every SM, down to the narrowest of the three-step pass on its lines
+  // (64^2, 4 coils, an apply alone 43.7 -> 38.5 us with the row passes' split above; 10
+  // iterations of CG on a few thousand pixels 10% faster)
+  const int64_t copies = stacked ? g.K : g.ncoils;
+  while (TC > (tiles ? lo : 2) && (g.inner() / TC) * copies < kSms) TC >>= 1;
+  return TC;
+}
+
 int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_shape, int K, int ncoils,
                      int precision, int kmax) {
   MRSR_REQUIRE(ndims == 2 || ndims == 3, MRSR_ERR_ARG, "ndims must be 2 or 3 (got %d)", ndims);
@@ -639,21 +678,7 @@ int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_
                  (long long)g.g[i]);
     MRSR_TRY(op->plan[i].init((int)g.g[i]));
   }
-  // Λ-pass tile width: up to 8 columns, a divisor of the plane width, <= 16384 elements per CTA
-  // generic kernels: two K*TC*L buffers; four-step kernels: one K*TC*L exchange buffer (<= ~110 KB, 2 CTAs/SM)
-  int TC = 8;
-  const int64_t budget = split_length((int)g.glast()) ? 13000 : 12288;
-  while (TC > 1 && ((int64_t)K * TC * g.glast() > budget || g.inner() % TC != 0)) TC >>= 1;
-  // narrower tiles where their CTAs (one per tile and coil, or per tile and plane of a stacked
-  // operator) would not reach every SM; 4 columns where the three-step pass takes the line
-  // (64^2, 4 coils, an apply alone 43.7 -> 38.5 us with the row passes' split below; 10
-  // iterations of CG on a few thousand pixels 10% faster)
-  const int64_t copies = kmax > KMAX ? K : ncoils;
-  const int tcmin = (g.glast() == 256 || g.glast() == 512) ? 4 : 2;
-  while (TC > tcmin && (g.inner() / TC) * copies < kSms) TC >>= 1;
-  // two CTAs of the three-step pass per SM: 28 KB of a line tile per component at 8 columns
-  if (g.glast() == 384 && K * TC > 28) TC = std::min(TC, 4);
-  op->TC = TC;
+  op->TC = lam_tile_width(op, kmax > KMAX);
   if (precision == MRSR_PREC_FP16_TC) {
     const int nl = (int)g.n[ndims - 1], gl = (int)g.glast();
     MRSR_REQUIRE(kind == MRSR_KIND_NFFT && tc_lambda_supported(gl, nl, nl, (int)g.inner(), K), MRSR_ERR_UNSUPPORTED,

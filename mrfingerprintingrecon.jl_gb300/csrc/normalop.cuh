@@ -115,6 +115,8 @@ int op_set_lambda_packed(mrsr_normalop* op, const void* lam_packed, int is_compl
                          int64_t nk, cudaStream_t st);
 // Λ of an FFT operator from the reference's full (K, K, grid...) complex array; kmask = Λ[1,1,:] .!= 0.
 int op_set_lambda_full(mrsr_normalop* op, const float2* lam_full, cudaStream_t st);
+// steps of the Λ pass's line transforms: 3 (apply_lam8.cu), 2 (a compiled split) or 0 (generic)
+int lam_pass_steps(const mrsr_normalop* op);
 // record op->last_use on `st` (the work enqueued so far on st may use op)
 int mark_use(const mrsr_normalop* op, cudaStream_t st);
 // marks the operator's use when the entry point returns

@@ -163,7 +163,11 @@ __device__ __forceinline__ void lam_apply(const LamPassArgs& a, int64_t lbase, i
 bool fast_length(int L);
 int fast_rows_fwd(const RowsFwdArgs& a, int64_t nrows, int ncg, cudaStream_t st);
 int fast_lambda(const LamPassArgs& a, int ncg, cudaStream_t st);
-// three-step Λ pass (apply_lam8.cu): 256- or 512-point lines pruned to half, 4- or 8-column tiles, K <= 6
+// three-step Λ pass (apply_lam8.cu): 256-, 384-, 512- and 768-point lines pruned to half, K <= kL8MaxK;
+// lambda8_tiles: the narrowest and the widest tile compiled for lines of L points, false if none
+constexpr int kL8MaxK = 6;
+bool lambda8_tiles(int L, int* lo, int* hi);
+bool lambda8_two_per_sm(int L, int TC, int K);  // whether two CTAs share an SM's shared memory
 bool lambda8_supported(const LamPassArgs& a);
 int fast_lambda8(const LamPassArgs& a, int ncg, cudaStream_t st);
 // three-step inverse row pass (apply_rows8.cu): 256- or 512-point rows of the zero-padded
