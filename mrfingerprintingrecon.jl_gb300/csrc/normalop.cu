@@ -477,10 +477,14 @@ static RowTiling rows_tiling(int L, int lines_per_row, int64_t nrows, int others
 }
 
 // Columns per CTA of the middle passes: 16 are 128-byte rows (128^3, 16 coils: the apply 11.49 ->
-// 10.65 ms against 8 columns; 32, one line each a CTA, 10.94); 8 for lines over 512 points, whose
-// two buffers of the generic kernel would not fit in shared memory at 16.
+// 10.65 ms against 8 columns; 32, one line each a CTA, 10.94); 8 for lines over 512 points and,
+// in the generic kernel, for those of which a CTA would not hold two rounds of 16: from 257 points
+// on its two buffers leave room for half the CTAs (64 x 243 x 64, K = 4, 8 coils, 486-point lines:
+// an apply 9.63 ms with 16 columns, 5.50 with 8; 64 x 375 x 64 Cartesian, K = 3, 8 coils, 1.88 and
+// 1.52 ms; 64 x 225 x 64, 0.993 and 0.983 ms; 64 x 125 x 64, K = 2, 0.365 and 0.377 ms).
 static int mid_tc(const mrsr_normalop* op) {
-  int TC = op->geo.g[1] <= 512 ? 16 : 8;
+  const int L = (int)op->geo.g[1];
+  int TC = (split_length(L) ? L <= 512 : 32 * L <= kMidElems) ? 16 : 8;
   while (TC > 1 && op->geo.g[0] % TC) TC >>= 1;
   return TC;
 }
