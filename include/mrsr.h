@@ -88,7 +88,9 @@ int mrsr_version(void);
  * ndims 2 or 3; img_shape host array; trj (ndims, ns_per_frame, nt);
  * sample_mask may be NULL (all samples); U (nt, K) real (u_is_complex = 0:
  * real kernel, ext:140) or complex (ext:89); cmaps may be NULL (one unit coil,
- * the reference's default cmaps=(1,)).  2*img_shape must be 2,3,5-smooth.
+ * the reference's default cmaps=(1,); ncoils is then the coil count of the
+ * operators that will share the kernel, which its layout is chosen for: 1 for
+ * none, 32 for any number).  2*img_shape must be 2,3,5-smooth.
  * Synchronous with respect to the host (it reads back sizes).
  */
 int mrsr_nfft_normalop_create(int ndims, const int64_t* img_shape, int64_t ns_per_frame, int64_t nt,
@@ -321,7 +323,10 @@ int mrsr_cg_relaxed(mrsr_normalop* op_lo, mrsr_normalop* op_hi, const float* b, 
  * which it shares by reference count (not copied), with its own coil maps
  * (cmaps (img..., ncoils) or NULL) and work stacks.  precision may differ
  * from src's (the fp16 copy of the kernel is made once and shared too).
- * Destroying src first is allowed.
+ * A float32 operator copies a kernel that is laid out for fewer coils, where
+ * its own layout has wider tiles (small images: the tiles of few coils are
+ * narrowed until they fill the GPU); a kernel made without maps for many
+ * coils (ncoils below) is never copied.  Destroying src first is allowed.
  */
 int mrsr_normalop_share(const mrsr_normalop* src, const float* cmaps, int ncoils, int precision,
                         mrsr_stream_t stream, mrsr_normalop** out);

@@ -386,6 +386,15 @@ bool half_supported(const mrsr_normalop* op) {
 }
 
 int half_lambda_convert(mrsr_normalop* op, cudaStream_t st) {
+  LamStore& store = *op->store;
+  DevBuf relaid;  // a shared kernel may have the tiles of the float32 passes
+  const float* lam = op->lam.as<float>();
+  if (op->TC != store.TC || op->FC != store.FC) {
+    MRSR_TRY(lam_relayout(op, op->TC, op->FC, op->P, relaid, st));
+    lam = relaid.as<float>();
+  }
+  store.half_TC = op->TC;
+  store.half_FC = op->FC;
   const int64_t per_tile = (int64_t)op->P * op->geo.glast() * op->TC * (op->lam_mode == LAM_PACKED_REAL ? 1 : 2);
   const int64_t ntiles = op->geo.inner() / op->TC;
   MRSR_TRY(op->lam_scale.alloc(sizeof(float) * ntiles));
@@ -394,10 +403,10 @@ int half_lambda_convert(mrsr_normalop* op, cudaStream_t st) {
   // tile max scaled to 1: the fp16-arithmetic (pair) kernels need |Λ| <= 1, the float32-arithmetic
   // ones take any scale, and operators of both kinds may share this copy
   const float target = 1.f;
-  k_lam_tile_max<<<b, 256, 0, st>>>(op->lam.as<float>(), per_tile, ntiles, target, op->lam_scale.as<float>());
+  k_lam_tile_max<<<b, 256, 0, st>>>(lam, per_tile, ntiles, target, op->lam_scale.as<float>());
   MRSR_LAUNCH_CHECK();
   const int64_t n = per_tile * ntiles;
-  k_lam_to_half<<<(unsigned)std::min<int64_t>(cdiv(n, 256), 65535), 256, 0, st>>>(op->lam.as<float>(), per_tile, n,
+  k_lam_to_half<<<(unsigned)std::min<int64_t>(cdiv(n, 256), 65535), 256, 0, st>>>(lam, per_tile, n,
                                                                                   op->lam_scale.as<float>(),
                                                                                   op->lam_half.as<__half>());
   MRSR_LAUNCH_CHECK();

@@ -214,7 +214,7 @@ extern "C" int mrsr_fft_normalop_create(int ndims, const int64_t* img_shape, int
   MRSR_REQUIRE(nrep >= 1 && ns_per_frame >= 1 && nt >= 1, MRSR_ERR_ARG, "empty trajectory");
   cudaStream_t st = cstream(stream);
   mrsr_normalop* op = new mrsr_normalop();
-  int s = op_init_geometry(op, MRSR_KIND_FFT, ndims, img_shape, K, cmaps ? ncoils : 1, precision);
+  int s = op_init_geometry(op, MRSR_KIND_FFT, ndims, img_shape, K, cmaps != nullptr, ncoils, precision);
   if (s == MRSR_OK) s = op_set_cmaps(op, cmaps, st);
   DevBuf acc;
   const int P = K * (K + 1) / 2;
@@ -246,7 +246,7 @@ extern "C" int mrsr_fft_normalop_create_from_mask(int ndims, const int64_t* img_
   MRSR_REQUIRE(M && U, MRSR_ERR_ARG, "M and U must be device pointers");
   cudaStream_t st = cstream(stream);
   mrsr_normalop* op = new mrsr_normalop();
-  int s = op_init_geometry(op, MRSR_KIND_FFT, ndims, img_shape, K, cmaps ? ncoils : 1, precision);
+  int s = op_init_geometry(op, MRSR_KIND_FFT, ndims, img_shape, K, cmaps != nullptr, ncoils, precision);
   if (s == MRSR_OK) s = op_set_cmaps(op, cmaps, st);
   DevBuf acc;
   const int P = K * (K + 1) / 2;

@@ -275,11 +275,11 @@ __global__ void k_lam_to_packed(LamLayout g, const T* lam, const int64_t* kmask,
   }
 }
 
-// the same rank-1 kernel in another chunked layout (P = 1 in both), every grid cell
+// the same kernel in another chunked layout, all P entries of every grid cell
 template <class T>
-__global__ void k_lam_relayout(LamLayout src, LamLayout dst, const T* a, T* b) {
+__global__ void k_lam_relayout(LamLayout src, LamLayout dst, int P, const T* a, T* b) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < dst.ngrid; c += (int64_t)gridDim.x * blockDim.x)
-    b[lam_int_index(dst, c, 0)] = a[lam_int_index(src, c, 0)];
+    for (int p = 0; p < P; ++p) b[lam_int_index(dst, c, p)] = a[lam_int_index(src, c, p)];
 }
 
 __global__ void k_flags_nonzero_c(const float2* lam_full, int64_t stride, int64_t n, uint8_t* flags) {
@@ -631,16 +631,15 @@ int normalop_apply_internal(mrsr_normalop* op, const float2* x, float2* y, float
 
 // Λ-pass tile width: up to 8 columns, a divisor of the plane width, <= 16384 elements per CTA
 // (generic kernels: two K*TC*L buffers; two-step kernels: one K*TC*L exchange buffer, <= ~110 KB,
-// two CTAs per SM), for the operator's coil count.
-static int lam_tile_width(const mrsr_normalop* op, bool stacked) {
-  const OpGeom& g = op->geo;
+// two CTAs per SM).
+int lam_tile_width(const OpGeom& g, int kind, int precision, bool stacked, int coils) {
   const int L = (int)g.glast();
   int TC = 8;
   const int64_t budget = split_length(L) ? 13000 : 12288;
   while (TC > 1 && ((int64_t)g.K * TC * L > budget || g.inner() % TC != 0)) TC >>= 1;
   int lo, hi;
   const bool tiles = lambda8_tiles(L, &lo, &hi);
-  const bool three = tiles && op->kind == MRSR_KIND_NFFT && op->precision == MRSR_PREC_FP32 && !stacked && g.K <= kL8MaxK;
+  const bool three = tiles && kind == MRSR_KIND_NFFT && precision == MRSR_PREC_FP32 && !stacked && g.K <= kL8MaxK;
   // the three-step pass: a compiled tile, narrow enough for two CTAs per SM (an apply of 384^2, 20
   // coils, K = 1 159 us with 8 columns, two-step, 129 with 4; K = 4 complex 585 us with 4, 529 with
   // 2; 256^2, 20 coils, K = 3 complex 159 us with 8, 137 with 4)
@@ -650,17 +649,17 @@ static int lam_tile_width(const mrsr_normalop* op, bool stacked) {
   // operator) would not reach every SM, down to the narrowest of the three-step pass on its lines
   // (64^2, 4 coils, an apply alone 43.7 -> 38.5 us with the row passes' split above; 10
   // iterations of CG on a few thousand pixels 10% faster)
-  const int64_t copies = stacked ? g.K : g.ncoils;
+  const int64_t copies = stacked ? g.K : coils;
   while (TC > (tiles ? lo : 2) && (g.inner() / TC) * copies < kSms) TC >>= 1;
   return TC;
 }
 
-int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_shape, int K, int ncoils,
+int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_shape, int K, bool maps, int ncoils,
                      int precision, int kmax) {
   MRSR_REQUIRE(ndims == 2 || ndims == 3, MRSR_ERR_ARG, "ndims must be 2 or 3 (got %d)", ndims);
   MRSR_REQUIRE(img_shape != nullptr, MRSR_ERR_ARG, "img_shape is NULL");
   MRSR_REQUIRE(K >= 1 && K <= kmax, MRSR_ERR_UNSUPPORTED, "rank K=%d outside 1..%d", K, kmax);
-  MRSR_REQUIRE(ncoils >= 1, MRSR_ERR_ARG, "ncoils must be >= 1");
+  MRSR_REQUIRE(!maps || ncoils >= 1, MRSR_ERR_ARG, "ncoils must be >= 1");
   MRSR_REQUIRE(precision == MRSR_PREC_FP32 || precision == MRSR_PREC_FP16 || precision == MRSR_PREC_FP16_TC, MRSR_ERR_ARG,
                "unknown precision %d",
                precision);
@@ -669,7 +668,7 @@ int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_
   OpGeom& g = op->geo;
   g.ndims = ndims;
   g.K = K;
-  g.ncoils = ncoils;
+  g.ncoils = maps ? ncoils : 1;
   for (int i = 0; i < 3; ++i) {
     g.n[i] = i < ndims ? img_shape[i] : 1;
     MRSR_REQUIRE(g.n[i] >= 1, MRSR_ERR_ARG, "image dimension %d must be positive", i + 1);
@@ -682,7 +681,7 @@ int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_
                  (long long)g.g[i]);
     MRSR_TRY(op->plan[i].init((int)g.g[i]));
   }
-  op->TC = lam_tile_width(op, kmax > KMAX);
+  op->TC = lam_tile_width(g, kind, precision, kmax > KMAX, std::max(ncoils, 1));
   if (precision == MRSR_PREC_FP16_TC) {
     const int nl = (int)g.n[ndims - 1], gl = (int)g.glast();
     MRSR_REQUIRE(kind == MRSR_KIND_NFFT && tc_lambda_supported(gl, nl, nl, (int)g.inner(), K), MRSR_ERR_UNSUPPORTED,
@@ -747,7 +746,8 @@ int op_finalize(mrsr_normalop* op, cudaStream_t st) {
     MRSR_TRY(tc_lambda_bound(op->lam.p, op->lam.bytes, op->lam_max.as<float>(), st));
     const size_t esz = op->lam_mode == LAM_PACKED_REAL ? sizeof(float) : sizeof(float2);
     MRSR_TRY(op->lam_tc.alloc(esz * (size_t)g.inner() * op->P * g.glast()));
-    MRSR_TRY(tc_lambda_layout(op->lam.p, op->lam_tc.p, g.inner(), op->P, op->FC, (int)(g.glast() / op->FC), op->TC,
+    const LamStore& s = *op->store;
+    MRSR_TRY(tc_lambda_layout(op->lam.p, op->lam_tc.p, g.inner(), op->P, s.FC, (int)(g.glast() / s.FC), s.TC,
                               op->lam_mode == LAM_PACKED_REAL, st));
   }
   // the operator's buffers came from the pool on `st`: make them usable on any stream
@@ -755,28 +755,61 @@ int op_finalize(mrsr_normalop* op, cudaStream_t st) {
   return MRSR_OK;
 }
 
+// layout of op->lam
 static LamLayout lam_layout(const mrsr_normalop* op) {
   LamLayout l;
   l.inner = op->geo.inner();
   l.L = op->geo.glast();
-  l.TC = op->TC;
+  l.TC = op->store->TC;
   l.P = op->P;
-  l.FC = op->FC;
-  l.NCH = (int)(l.L / op->FC);
+  l.FC = op->store->FC;
+  l.NCH = (int)(l.L / l.FC);
   l.ngrid = op->geo.ngrid();
   return l;
+}
+
+int lam_relayout(const mrsr_normalop* src, int TC, int FC, int P, DevBuf& out, cudaStream_t st) {
+  const LamLayout ls = lam_layout(src);
+  LamLayout ld = ls;
+  ld.TC = TC;
+  ld.FC = FC;
+  ld.NCH = (int)(ls.L / FC);
+  const bool real = lam_is_real(src->lam_mode);
+  MRSR_TRY(out.alloc((real ? sizeof(float) : sizeof(float2)) * (size_t)P * ls.ngrid));
+  const unsigned blocks = (unsigned)std::min<int64_t>(cdiv(ls.ngrid, 256), 65535);
+  if (real)
+    k_lam_relayout<float><<<blocks, 256, 0, st>>>(ls, ld, P, src->lam.as<float>(), out.as<float>());
+  else
+    k_lam_relayout<float2><<<blocks, 256, 0, st>>>(ls, ld, P, src->lam.as<float2>(), out.as<float2>());
+  MRSR_LAUNCH_CHECK();
+  return MRSR_OK;
 }
 
 // Λ chunk length: the largest divisor of L with at most 256 positions (FC * TC), so the entries
 // of neighbouring frequencies and columns lie together.  The three-step pass wants all 256, also
 // where a chunk of a large kernel is over 16 KB (128^2, K = 6, 16 coils, an apply 63.9 -> 58.5 us;
 // 256^2 complex, K = 5, 20 coils 270 -> 221).
-static void choose_fc(mrsr_normalop* op) {
-  const int L = (int)op->geo.glast();
+int lam_chunk(int64_t L, int TC) {
   int best = 1;
   for (int fc = 1; fc <= L; ++fc)
-    if (L % fc == 0 && (int64_t)fc * op->TC <= 256) best = fc;
-  op->FC = best;
+    if (L % fc == 0 && (int64_t)fc * TC <= 256) best = fc;
+  return best;
+}
+
+// the operator's own kernel, in the layout of its tile width
+static void own_layout(mrsr_normalop* op) {
+  op->FC = lam_chunk(op->geo.glast(), op->TC);
+  op->store->TC = op->TC;
+  op->store->FC = op->FC;
+}
+
+int op_copy_kernel(mrsr_normalop* op, const mrsr_normalop* src, cudaStream_t st) {
+  op->nk = src->nk;
+  own_layout(op);
+  MRSR_TRY(lam_relayout(src, op->TC, op->FC, op->P, op->lam, st));
+  MRSR_TRY(op->kmask.alloc(sizeof(int64_t) * (size_t)src->nk));
+  MRSR_CHECK_CUDA(cudaMemcpyAsync(op->kmask.p, src->kmask.p, sizeof(int64_t) * src->nk, cudaMemcpyDeviceToDevice, st));
+  return MRSR_OK;
 }
 
 int op_set_lambda_packed(mrsr_normalop* op, const void* lam_packed, int is_complex, const int64_t* kmask, int64_t nk,
@@ -787,7 +820,7 @@ int op_set_lambda_packed(mrsr_normalop* op, const void* lam_packed, int is_compl
   op->lam_mode = is_complex ? LAM_PACKED_CPLX : LAM_PACKED_REAL;
   op->P = K * (K + 1) / 2;
   op->nk = nk;
-  choose_fc(op);
+  own_layout(op);
   const size_t esz = is_complex ? sizeof(float2) : sizeof(float);
   MRSR_TRY(op->lam.alloc(esz * op->P * op->geo.ngrid()));
   MRSR_CHECK_CUDA(cudaMemsetAsync(op->lam.p, 0, op->lam.bytes, st));
@@ -825,7 +858,7 @@ int op_set_lambda_full(mrsr_normalop* op, const float2* lam_full, cudaStream_t s
   op->lam_mode = LAM_FULL_CPLX;
   op->P = K * K;
   op->nk = nk;
-  choose_fc(op);
+  own_layout(op);
   MRSR_TRY(op->lam.alloc(sizeof(float2) * op->P * ng));
   MRSR_CHECK_CUDA(cudaMemsetAsync(op->lam.p, 0, op->lam.bytes, st));
   DevBuf packed;
@@ -859,7 +892,7 @@ extern "C" int mrsr_nfft_normalop_from_lambda(int ndims, const int64_t* img_shap
   *out = nullptr;
   cudaStream_t st = as_stream(stream);
   mrsr_normalop* op = new mrsr_normalop();
-  int s = op_init_geometry(op, MRSR_KIND_NFFT, ndims, img_shape, K, cmaps ? ncoils : 1, precision);
+  int s = op_init_geometry(op, MRSR_KIND_NFFT, ndims, img_shape, K, cmaps != nullptr, ncoils, precision);
   if (s == MRSR_OK) s = op_set_cmaps(op, cmaps, st);
   if (s == MRSR_OK) s = op_set_lambda_packed(op, lambda_packed, lambda_is_complex, kmask_indcs, nk, st);
   if (s == MRSR_OK) s = op_finalize(op, st);
@@ -880,7 +913,7 @@ extern "C" int mrsr_fft_normalop_from_lambda(int ndims, const int64_t* img_shape
   MRSR_REQUIRE(lambda_full, MRSR_ERR_ARG, "Λ is NULL");
   cudaStream_t st = as_stream(stream);
   mrsr_normalop* op = new mrsr_normalop();
-  int s = op_init_geometry(op, MRSR_KIND_FFT, ndims, img_shape, K, cmaps ? ncoils : 1, precision);
+  int s = op_init_geometry(op, MRSR_KIND_FFT, ndims, img_shape, K, cmaps != nullptr, ncoils, precision);
   if (s == MRSR_OK) s = op_set_cmaps(op, cmaps, st);
   if (s == MRSR_OK) s = op_set_lambda_full(op, reinterpret_cast<const float2*>(lambda_full), st);
   if (s == MRSR_OK) s = op_finalize(op, st);
@@ -1080,34 +1113,11 @@ extern "C" int mrsr_normalop_stack(const mrsr_normalop* src, int nrhs, mrsr_stre
                (long long)lmax);
   cudaStream_t st = as_stream(stream);
   mrsr_normalop* op = new mrsr_normalop();
-  int s = op_init_geometry(op, src->kind, g.ndims, g.n, nrhs, g.ncoils, MRSR_PREC_FP32, kStackMax);
+  int s = op_init_geometry(op, src->kind, g.ndims, g.n, nrhs, src->cmaps.p != nullptr, g.ncoils, MRSR_PREC_FP32, kStackMax);
   if (s == MRSR_OK) {
-    const bool real = lam_is_real(src->lam_mode);
-    op->lam_mode = real ? LAM_DIAG_REAL : LAM_DIAG_CPLX;
+    op->lam_mode = lam_is_real(src->lam_mode) ? LAM_DIAG_REAL : LAM_DIAG_CPLX;
     op->P = 1;
-    op->nk = src->nk;
-    choose_fc(op);
-    const size_t esz = real ? sizeof(float) : sizeof(float2);
-    s = op->lam.alloc(esz * (size_t)g.ngrid());
-    if (s == MRSR_OK) {
-      const LamLayout ls = lam_layout(src), ld = lam_layout(op);
-      const unsigned blocks = (unsigned)std::min<int64_t>(cdiv(g.ngrid(), 256), 65535);
-      if (real)
-        k_lam_relayout<float><<<blocks, 256, 0, st>>>(ls, ld, src->lam.as<float>(), op->lam.as<float>());
-      else
-        k_lam_relayout<float2><<<blocks, 256, 0, st>>>(ls, ld, src->lam.as<float2>(), op->lam.as<float2>());
-      if (cudaGetLastError() != cudaSuccess) {
-        set_error("Λ relayout launch failed");
-        s = MRSR_ERR_CUDA;
-      }
-    }
-    if (s == MRSR_OK) s = op->kmask.alloc(sizeof(int64_t) * (size_t)src->nk);
-    if (s == MRSR_OK &&
-        cudaMemcpyAsync(op->kmask.p, src->kmask.p, sizeof(int64_t) * src->nk, cudaMemcpyDeviceToDevice, st) !=
-            cudaSuccess) {
-      set_error("kmask copy failed");
-      s = MRSR_ERR_CUDA;
-    }
+    s = op_copy_kernel(op, src, st);
     if (s == MRSR_OK && src->cmaps.p) s = op_set_cmaps(op, src->cmaps.as<float>(), st);
   }
   if (s == MRSR_OK) s = op_finalize(op, st);

@@ -40,8 +40,10 @@ struct OpGeom {
 struct LamStore {
   DevBuf kmask;      // int64 nk, 1-based column-major grid indices
   DevBuf lam;        // [tile][chunk][P][FC][TC] of float / float2 (chunked along f_last)
+  int TC = 0, FC = 0;            // layout of lam
   DevBuf lam_scale;  // fp16: one float per tile
   DevBuf lam_half;   // fp16: the chunked kernel in half precision
+  int half_TC = 0, half_FC = 0;  // layout of lam_half
   DevBuf lam_max;    // fp16-tc: largest |component| of Λ (float)
   DevBuf lam_tc;     // fp16-tc: Λ rearranged for the tensor-core Λ pass
   DevBuf tc_consts;  // fp16-tc: DFT-64 MMA operand and twiddles
@@ -104,12 +106,22 @@ struct mrsr_normalop {
 
 namespace mrsr {
 // Build helpers shared by the constructors (normalop.cu).
-// kmax: the largest K accepted (the rank limit of the K x K contraction unless the
-// operator is a stacked one, whose planes are independent)
-int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_shape, int K,
+// maps: whether the operator has coil maps (`ncoils` of them; without, it has one unit coil and
+// ncoils is the coil count its kernel is laid out for).  kmax: the largest K accepted (the rank
+// limit of the K x K contraction unless the operator is a stacked one, whose planes are independent)
+int op_init_geometry(mrsr_normalop* op, int kind, int ndims, const int64_t* img_shape, int K, bool maps,
                      int ncoils, int precision, int kmax = 8);
+constexpr int kManyCoils = 32;  // coils a kernel is laid out for that serves any number of them
+// columns per tile of the Λ pass for `coils` coils
+int lam_tile_width(const OpGeom& g, int kind, int precision, bool stacked, int coils);
+// largest chunk length of a layout with TC columns per tile
+int lam_chunk(int64_t L, int TC);
+// the kernel of `src` in the layout (TC, FC), P entries per cell
+int lam_relayout(const mrsr_normalop* src, int TC, int FC, int P, DevBuf& out, cudaStream_t st);
 int op_set_cmaps(mrsr_normalop* op, const float* cmaps, cudaStream_t st);
 int op_finalize(mrsr_normalop* op, cudaStream_t st);
+// kernel and kmask of `src`, copied into the layout of op's tile width (lam_mode and P are op's)
+int op_copy_kernel(mrsr_normalop* op, const mrsr_normalop* src, cudaStream_t st);
 // Λ from the reference's packed (P, nk) layout at 1-based kmask cells.
 int op_set_lambda_packed(mrsr_normalop* op, const void* lam_packed, int is_complex, const int64_t* kmask,
                          int64_t nk, cudaStream_t st);

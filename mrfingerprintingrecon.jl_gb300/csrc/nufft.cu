@@ -1558,7 +1558,7 @@ extern "C" int mrsr_nfft_normalop_create(int ndims, const int64_t* img_shape, in
   MRSR_REQUIRE(ns_per_frame >= 1 && nt >= 1, MRSR_ERR_ARG, "empty trajectory");
   cudaStream_t st = nstream(stream);
   mrsr_normalop* op = new mrsr_normalop();
-  int s = op_init_geometry(op, MRSR_KIND_NFFT, ndims, img_shape, K, cmaps ? ncoils : 1, precision);
+  int s = op_init_geometry(op, MRSR_KIND_NFFT, ndims, img_shape, K, cmaps != nullptr, ncoils, precision);
   if (s == MRSR_OK) s = op_set_cmaps(op, cmaps, st);
   SampleList sl;
   DevBuf kmask, packed;

@@ -1,8 +1,8 @@
 // Pieces of the reconstruction server that live below the C ABI:
 //
 // * mrsr_normalop_share: a new operator on an existing operator's Toeplitz
-//   kernel and kmask (held by reference count, never copied) with its own coil
-//   maps and work stacks.  A server keeps one kernel per trajectory and basis
+//   kernel and kmask (held by reference count, and copied only from a kernel laid
+//   out for fewer coils) with its own coil maps and work stacks.  A server keeps one kernel per trajectory and basis
 //   and makes a cheap operator per request from it.
 // * mrsr_cg_batch_*: fixed-iteration CG solves of several independent systems
 //   recorded once into one CUDA graph, one branch per system, so a batch is a
@@ -88,16 +88,31 @@ extern "C" int mrsr_normalop_share(const mrsr_normalop* src, const float* cmaps,
   MRSR_REQUIRE(src, MRSR_ERR_ARG, "source operator is NULL");
   MRSR_REQUIRE(src->lam.p && src->kmask.p, MRSR_ERR_STATE, "source operator has no kernel");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  mrsr_normalop* op = new mrsr_normalop(src->store);
   const OpGeom& g = src->geo;
-  int s = op_init_geometry(op, src->kind, g.ndims, g.n, g.K, cmaps ? ncoils : 1, precision);
+  // the fp16 copy is made once for all coil counts
+  const int nc = std::max(ncoils, precision == MRSR_PREC_FP16 ? kManyCoils : 1);
+  const int TC = lam_tile_width(g, src->kind, precision, lam_is_diag(src->lam_mode), nc);
+  // A kernel laid out for fewer coils has tiles too narrow for this operator: a float32 operator
+  // then takes a copy in its own layout.  (256^2, K = 2, 20 coils on the layout for one coil,
+  // 4 columns, an apply 91.5 us; on its own, 8 columns, 85.5.)
+  const bool copy = precision == MRSR_PREC_FP32 && TC > src->store->TC;
+  mrsr_normalop* op = copy ? new mrsr_normalop() : new mrsr_normalop(src->store);
+  int s = op_init_geometry(op, src->kind, g.ndims, g.n, g.K, cmaps != nullptr, ncoils, precision);
   if (s == MRSR_OK) {
     op->lam_mode = src->lam_mode;
     op->P = src->P;
     op->nk = src->nk;
-    op->TC = src->TC;
-    op->FC = src->FC;
-    s = op_set_cmaps(op, cmaps, st);
+    const LamStore& store = *src->store;
+    if (copy) {
+      s = op_copy_kernel(op, src, st);
+    } else if (precision == MRSR_PREC_FP16) {
+      op->TC = store.lam_half.p ? store.half_TC : TC;
+      op->FC = store.lam_half.p ? store.half_FC : lam_chunk(g.glast(), TC);
+    } else {
+      op->TC = store.TC;
+      op->FC = store.FC;
+    }
+    if (s == MRSR_OK) s = op_set_cmaps(op, cmaps, st);
   }
   if (s == MRSR_OK) s = op_finalize(op, st);
   if (s != MRSR_OK) {

@@ -147,7 +147,8 @@ class NormalOperator:
     Lambda = Λ
 
     def share(self, cmaps=None, precision=None, stream=None):
-        """A new operator on this operator's Toeplitz kernel and kmask (shared, not copied)
+        """A new operator on this operator's Toeplitz kernel and kmask (shared; copied only where this
+        operator's layout is for fewer coils, see ``shared`` of :func:`NFFTNormalOp`)
         with its own coil maps; ``precision`` defaults to this operator's."""
         S = stack_cmaps(cmaps)
         nc = 1 if S is None else int(S.shape[-1])
@@ -192,18 +193,20 @@ def _img(img_shape):
 
 
 def NFFTNormalOp(img_shape, trj_or_lambda, U_or_kmask, cmaps=None, sample_mask=None, precision="fp32",
-                 stream=None):
+                 stream=None, shared=False):
     """``NFFTNormalOp(img_shape, trj, U; cmaps, sample_mask)`` or
     ``NFFTNormalOp(img_shape, Λ, kmask_indcs; cmaps)`` (packed GPU Λ).
 
     trj: (d, Ns, Nt) float32 in [-0.5, 0.5]; U: (Nt, K) real or complex.
     Λ: packed (K(K+1)/2, Nk) float32 or complex64; kmask_indcs: 1-based int64.
+    ``shared`` (without coil maps): lay the kernel out for the operators that will share it with
+    maps (:meth:`NormalOperator.share`) rather than for this operator's one coil.
     """
     lib = _lib.load()
     img_shape = _img(img_shape)
     d = len(img_shape)
     S = stack_cmaps(cmaps, img_shape)
-    nc = 1 if S is None else int(S.shape[-1])
+    nc = (32 if shared else 1) if S is None else int(S.shape[-1])
     arr = trj_or_lambda
     is_traj = (getattr(arr, "ndim", None) or getattr(arr, "dim", lambda: 0)()) in (3, 4) and arr.shape[0] == d
     if is_traj:

@@ -378,7 +378,7 @@ class GpuExecutor:
     def build_kernel(self, proto, si):
         s = self._stream(si)
         with self.torch.cuda.stream(s):
-            return self.mr.NFFTNormalOp(proto.img, proto.trj, proto.U, stream=s)
+            return self.mr.NFFTNormalOp(proto.img, proto.trj, proto.U, stream=s, shared=True)
 
     def drop_kernel(self, kern):
         kern.close()
