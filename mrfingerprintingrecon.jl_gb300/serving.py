@@ -116,6 +116,15 @@ def kernel_bytes(img, K, nk=None, complex_kernel=False, fp16=False, tc=False):
     return lam + half + tcl + 8 * nk + base_stack
 
 
+def spread_parts(parts):
+    """Accumulators of a backprojection of `parts` real planes: padded to the lanes of their groups (8, 16 or
+    32, as spread_lanes in csrc/spread_rows.cuh picks them)."""
+    if parts <= 8:
+        return 8
+    padded = {p: -(-parts // p) * p for p in (32, 16)}
+    return min(padded.items(), key=lambda e: e[1] * (7 + 32 // e[0]))[1]
+
+
 def request_bytes(img, K, nc, precision="fp32", refine=False):
     """Device bytes one admitted request holds while it runs (estimate, rounded up)."""
     img = tuple(int(v) for v in img)
@@ -131,8 +140,9 @@ def request_bytes(img, K, nc, precision="fp32", refine=False):
     ops = stacks + nimg * nc * 8
     if refine:
         ops *= 2
-    # backprojection: float2 grid plus its 64-bit fixed-point accumulator (re, im) per coil batch
-    bp_grid = 3 * K * G * 8 * min(nc, max(1, (2 << 30) // (K * G * 8)))
+    # backprojection: float2 grid plus its 64-bit fixed-point accumulators (re, im) per coil batch
+    cb = min(nc, max(1, (2 << 30) // (K * G * 8)))
+    bp_grid = G * 8 * (K * cb + spread_parts(2 * K * cb))
     cgwork = 3 * vec + 32 * 1024
     return int(1.1 * (ops + bp_grid + cgwork + 2 * vec + (2 * vec if refine else 0))) + (1 << 20)
 
