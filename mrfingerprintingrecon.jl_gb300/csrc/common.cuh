@@ -50,9 +50,11 @@ struct Status {
 // memory comes from the stream-ordered pool (cudaMallocAsync) on the call's
 // stream, so the library never calls cudaMalloc / cudaFree, which would
 // synchronise the whole device and stall other streams' work.  A buffer released
-// inside a call is freed on the call's stream; one released with its operator, on
-// the library's private stream after that stream has waited for the operator's
-// last use (see mrsr_normalop).
+// inside a call is freed on the call's stream (or, marked `side`, on the private
+// stream after the call's work); one released with its operator, on the library's
+// private stream after that stream has waited for the operator's last use (see
+// mrsr_normalop).
+constexpr uint64_t kPoolKeep = 8ull << 30;  // freed bytes that the pool keeps for reuse
 cudaStream_t lib_stream();          // private non-blocking stream of the current device
 cudaStream_t call_stream();         // stream of the running entry point, else lib_stream()
 bool in_call();
@@ -72,6 +74,7 @@ struct CallScope {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool side = false;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;

@@ -1067,6 +1067,10 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   MRSR_TRY(grid.alloc(sizeof(float2) * mcells * pb));
   MRSR_TRY(qgrid.alloc(qbytes));
   MRSR_TRY(cgrid.alloc(sizeof(float2) * gcells * P));
+  // The call synchronises after these are freed.  Where they are more than the pool keeps, freed on
+  // the call's stream they went back to the driver there, and the next call mapped them anew (192^3,
+  // K = 3, calls in a row 129 ms against 88; 128^3, K = 5, 72 against 67).
+  grid.side = qgrid.side = cgrid.side = grid.bytes + qgrid.bytes + cgrid.bytes > kPoolKeep;
   // fixed-point scale: |term| <= (2 if complex) max|U|^2 (the kernel taps are <= 1), and a cell
   // of the upsampled grid gets at most ceil(w / M) taps per sample and dimension
   MRSR_TRY(fsb.alloc(sizeof(FixedScale)));

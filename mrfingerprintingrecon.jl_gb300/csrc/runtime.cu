@@ -10,6 +10,7 @@ namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 cudaStream_t g_lib[kMaxDevices] = {nullptr};
+cudaEvent_t g_fence[kMaxDevices] = {nullptr};
 thread_local cudaStream_t t_call = nullptr;
 thread_local bool t_in_call = false;
 
@@ -19,15 +20,15 @@ int current_device() {
   return d;
 }
 
-// first use on a device: the private stream, and a pool that keeps up to 32 GiB of freed blocks for
-// reuse (the grids of a kernel precompute up to 192^3; with 8 GiB each of its calls mapped memory
-// anew: 192^3, K = 3, 137 ms against 87, 128^3, K = 5, 94 against 87) and never makes one stream
-// wait on another to hand a block over
+// first use on a device: the private stream, and a pool that keeps up to 8 GiB of freed blocks
+// for reuse (the rest of the process shares the device's default pool and its memory) and never
+// makes one stream wait on another to hand a block over
 void init_device(int d) {
   cudaStreamCreateWithFlags(&g_lib[d], cudaStreamNonBlocking);
+  cudaEventCreateWithFlags(&g_fence[d], cudaEventDisableTiming);
   cudaMemPool_t pool;
   if (cudaDeviceGetDefaultMemPool(&pool, d) == cudaSuccess) {
-    uint64_t keep = 32ull << 30;
+    uint64_t keep = kPoolKeep;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     int no = 0;
     cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no);
@@ -61,12 +62,22 @@ CallScope::~CallScope() {
   t_in_call = prev_in;
 }
 
+// lib_stream() waits for the work enqueued so far on `s`
+static bool fence_lib_after(cudaStream_t s) {
+  cudaStream_t ls = lib_stream();
+  const int d = current_device();
+  std::lock_guard<std::mutex> lock(g_mu);  // one fence event per device, reused under the lock
+  return cudaEventRecord(g_fence[d], s) == cudaSuccess && cudaStreamWaitEvent(ls, g_fence[d], 0) == cudaSuccess;
+}
+
 // Inside a call the block goes back on the call's own stream: the next call on that stream
 // takes it again without waiting for it (freed on another stream, it is out of reach until the
-// GPU has got there, and calls in a row without a synchronisation made the pool grow).
+// GPU has got there, and calls in a row without a synchronisation made the pool grow).  A `side`
+// block goes back on the private stream behind the call's work.
 void DevBuf::release() {
   if (!p) return;
-  cudaFreeAsync(p, t_in_call ? t_call : lib_stream());
+  const bool on_call = t_in_call && !(side && fence_lib_after(t_call));
+  cudaFreeAsync(p, on_call ? t_call : lib_stream());
   p = nullptr;
   bytes = 0;
 }
