@@ -20,6 +20,7 @@
 #include <cstring>
 #include <vector>
 
+#include "fft4.cuh"
 #include "passes.cuh"
 #include "splits.cuh"
 
@@ -704,6 +705,12 @@ int op_set_cmaps(mrsr_normalop* op, const float* cmaps, cudaStream_t st) {
   return MRSR_OK;
 }
 
+// shared memory of one coil's row in the inverse row pass
+static int64_t rows_inv_line_bytes(int L) {
+  const int r1 = split_r1(L);
+  return (int64_t)sizeof(float2) * (r1 ? r1 * slots_width(L / r1, 1) : 2 * L);
+}
+
 int op_finalize(mrsr_normalop* op, cudaStream_t st) {
   const OpGeom& g = op->geo;
   const bool half = op->precision == MRSR_PREC_FP16;
@@ -723,8 +730,10 @@ int op_finalize(mrsr_normalop* op, cudaStream_t st) {
     const int64_t per_coil3 = per_coil + (int64_t)g.K * g.g[0] * g.g[1] * g.n[2] * esz;
     cg = std::max<int64_t>(1, (12288ll << 20) / std::max<int64_t>(per_coil3, 1));
   }
-  // rows inverse holds one row of every coil of the group in shared memory (<= ~200 KB)
+  // rows inverse holds one row of every coil of the group in shared memory (<= ~200 KB, and no more
+  // than a block can have with the padding of the row's split or the generic kernel's two buffers)
   cg = std::min<int64_t>(cg, std::max<int64_t>(1, (200ll << 10) / (9 * g.g[0])));
+  if (!half) cg = std::min<int64_t>(cg, std::max<int64_t>(1, ((227ll << 10) - 8 * g.g[0]) / rows_inv_line_bytes((int)g.g[0])));
   cg = std::min<int64_t>(cg, g.ncoils);
   const int64_t ngroups = cdiv(g.ncoils, cg);
   cg = cdiv(g.ncoils, ngroups);
