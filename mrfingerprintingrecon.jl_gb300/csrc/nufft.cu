@@ -1062,7 +1062,7 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   const bool tiled = S.n < (1ll << 31) && S.ns_pf * S.nt < (1ll << 31);
   const bool rows = tiled && (d == 2 || rows_pay(nq * pb, nq * P, S.n, mcells));
   if (d == 3 && !rows) pb = std::max(pb, std::min(P, kP3 / nq));
-  DevBuf grid, qgrid, cgrid, fsb, umax, bad;
+  DevBuf grid, qgrid, cgrid, fsb, umax;
   const size_t qbytes = rows ? spread_rows_bytes(nq * pb, mcells) : sizeof(long long) * nq * mcells * pb;
   MRSR_TRY(grid.alloc(sizeof(float2) * mcells * pb));
   MRSR_TRY(qgrid.alloc(qbytes));
@@ -1086,22 +1086,20 @@ static int compute_lambda(int d, const int64_t* G, const SampleSet& S, const voi
   if (tiled || ordered) MRSR_TRY(ts.build(S, M, rows ? kSpTile : kTile3, rows ? spread_chunk(d, S.n) : kChunk, rows, st));
   if (tiled) MRSR_TRY(ts.prep(S, MRSR_DCF_NONE, nullptr, st));
   if (rows) {
-    MRSR_TRY(umax.alloc(sizeof(float) * K));
-    MRSR_TRY(bad.alloc(sizeof(int) * nq * pb));
-    k_basis_max<<<K, 256, 0, st>>>(U, S.nt, u_complex, umax.as<float>());
-    MRSR_LAUNCH_CHECK();
+    MRSR_TRY(basis_max(S, U, u_complex, K, nq * P, umax, st));
   }
   const TileSort* tsp = tiled || ordered ? &ts : nullptr;
   MRSR_TRY(packed.alloc((u_complex ? 8 : 4) * (size_t)P * std::max<int64_t>(*nk_out, 1)));
   // channels in batches of pb: spread, inverse DFT on the upsampled grid, deconvolve and fold onto the 2x grid
   for (int p0 = 0; p0 < P; p0 += pb) {
     const int np = std::min(pb, P - p0);
+    int* bad = rows ? umax.as<int>() + K + nq * p0 : nullptr;
     MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, rows ? spread_rows_bytes(nq * np, mcells) : sizeof(long long) * nq * mcells * np, st));
     SpreadLambdaArgs sa{S, {M[0], M[1], M[2]}, mcells, U, u_complex, K, P, p0, np, nq, qgrid.as<long long>(),
-                        fsb.as<FixedScale>(), umax.as<float>(), bad.as<int>()};
+                        fsb.as<FixedScale>(), umax.as<float>(), bad};
     MRSR_TRY(spread_lambda(sa, tsp, st));
     if (rows)
-      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), nq, mcells, nq * np, fsb.as<FixedScale>(), bad.as<int>(), grid.as<float2>(),
+      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), nq, mcells, nq * np, fsb.as<FixedScale>(), bad, grid.as<float2>(),
                              st));
     else
       MRSR_TRY(fixed_to_grid(qgrid.as<long long>(), nq, mcells, np, fsb.as<FixedScale>(), grid.as<float2>(), st));
@@ -1648,28 +1646,26 @@ extern "C" int mrsr_backprojection(int ndims, const int64_t* img_shape, int64_t 
     MRSR_TRY(fixed_scale(f, n, nf, mult, (double)sl.set.n * taps_per_cell(ndims, M), rows, fsb.as<FixedScale>(), st));
   }
   TileSort ts;
-  DevBuf umax, tmax, bad;
+  DevBuf umax, tmax;
   const bool ordered = ndims == 3 && sl.set.n < (1ll << 31);
   if (tiled || ordered) MRSR_TRY(ts.build(sl.set, M, rows ? kSpTile : kTile3, rows ? spread_chunk(ndims, sl.set.n) : kChunk, rows, st));
   if (tiled) MRSR_TRY(ts.prep(sl.set, dcf_kind, dcf_array, st));
   if (rows) {
-    MRSR_TRY(umax.alloc(sizeof(float) * K));
     MRSR_TRY(tmax.alloc(sizeof(float) * (size_t)ts.ntiles * cc));
-    MRSR_TRY(bad.alloc(sizeof(int) * 2 * K * cc));
-    k_basis_max<<<K, 256, 0, st>>>(U, nt, u_is_complex, umax.as<float>());
-    MRSR_LAUNCH_CHECK();
+    MRSR_TRY(basis_max(sl.set, U, u_is_complex, K, 2 * K * ncoils, umax, st));
   }
   const int64_t out_elems = nimg * K * (cmaps ? 1 : ncoils);
   if (cmaps) MRSR_CHECK_CUDA(cudaMemsetAsync(out, 0, sizeof(float2) * out_elems, st));
   for (int c0 = 0; c0 < ncoils; c0 += cc) {
     const int nc = std::min(cc, ncoils - c0);
+    int* bad = rows ? umax.as<int>() + K + 2 * K * c0 : nullptr;
     MRSR_CHECK_CUDA(cudaMemsetAsync(qgrid.p, 0, rows ? spread_rows_bytes(2 * K * nc, mcells) : (size_t)per_coil * 2 * nc, st));
     SpreadDataArgs sa{sl.set, {M[0], M[1], M[2]}, mcells, reinterpret_cast<const float2*>(data), c0, nc, U,
                       u_is_complex, K, dcf_kind, dcf_array, qgrid.as<long long>(), fsb.as<FixedScale>(), umax.as<float>(),
-                      tmax.as<float>(), bad.as<int>()};
+                      tmax.as<float>(), bad};
     MRSR_TRY(spread_data(sa, tiled || ordered ? &ts : nullptr, st));
     if (rows) {
-      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), 2, mcells, 2 * K * nc, fsb.as<FixedScale>(), bad.as<int>(),
+      MRSR_TRY(parts_to_grid(qgrid.as<long long>(), 2, mcells, 2 * K * nc, fsb.as<FixedScale>(), bad,
                              grid.as<float2>(), st));
     } else if (parts_layout) {
       k_fixed_to_grid_cp<<<(unsigned)cdiv(mcells, 32), 256, 0, st>>>(qgrid.as<long long>(), 2 * nc * K, mcells,

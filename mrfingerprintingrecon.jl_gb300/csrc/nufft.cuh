@@ -142,7 +142,7 @@ struct SpreadLambdaArgs {
   long long* q;       // [np][nq][cells], or the parts layout of spread_rows.cuh on its tiles
   const FixedScale* fs;
   const float* umax;  // with tap records: k_basis_max of U
-  int* bad;           // and room for a mark per part (spread_rows.cuh)
+  int* bad;           // and the parts' marks (spread_rows.cuh)
 };
 // Samples of a set counting-sorted by the tile (`tile` cells a side) of the grid M that holds
 // their first tap, in chunks (the work items of the tile-sorted kernels) of at most `most`
@@ -176,7 +176,7 @@ struct SpreadDataArgs {
   const FixedScale* fs;
   const float* umax;    // with tap records: k_basis_max of U, and room for ntiles * nc maxima
   float* tmax;
-  int* bad;             // and for a mark per part (spread_rows.cuh)
+  int* bad;             // and the parts' marks (spread_rows.cuh)
 };
 int spread_data(const SpreadDataArgs& a, const TileSort* ts, cudaStream_t st);
 

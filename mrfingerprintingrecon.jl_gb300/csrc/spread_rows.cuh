@@ -21,9 +21,11 @@
 // 64-bit sums as those of terms rounded to 2^-40 of the largest one (1.6e-7 on 256^2, 512k
 // samples, 20 coils; with 27 bits for the values instead of 29, 1.7e-7).
 //
-// An integer cannot hold an infinity or a NaN, so a value that is not finite marks its part in
-// `bad`, and the conversion to float makes every cell of a marked part NaN, as a float sum's
-// transform would be.  The maxima run over finite entries, so the other parts are untouched.
+// An integer cannot hold an infinity or a NaN, so the maxima (which run over the samples and
+// frames that are used) are infinite where one of their entries is not finite.  Such a bound marks
+// its part in `bad`, and the conversion to float makes every cell of a marked part NaN, as a float
+// sum's transform would be.  (A check of every value instead took 4% of the backprojection of
+// 256^2, 20 coils.)
 //
 // 256^2, 512k samples, 20 coils, K = 5 (200 parts): 1.51 ms against 2.93 ms for windows of 32-bit
 // limbs in shared memory, two shared atomics and about eight instructions per term; the 15
@@ -55,7 +57,7 @@ struct SpreadRowsArgs {
   int nparts;              // parts to spread
   long long* q;            // [ceil(nparts / P)][cells][P]
   const FixedScale* fs;
-  int* bad;                // [nparts], zeroed: set for parts that hold a value that is not finite
+  int* bad;                // [nparts], cleared by k_basis_max: set for parts that hold a value that is not finite
   int ntx, nty;
   const void* rec;         // TapRec (2D) or TapRec3 (3D) in sorted order
   const int4* items;       // (tile, first sorted position, count, -)
@@ -63,9 +65,13 @@ struct SpreadRowsArgs {
   unsigned long long* next;  // work counter, zeroed before the launch
 };
 
+// bound of a product of two values from their bounds: NaN if one of them is not finite
+__device__ __forceinline__ float part_bound(float a, float b) {
+  return finite_value(a) && finite_value(b) ? fminf(a * b, kFltMax) : __int_as_float(0x7fc00000);
+}
+
 // Part p of the Λ precompute: pair p0 + p / nq (k1 <= k2, packed k2 (k2 + 1) / 2 + k1), plane
-// p % nq; value conj(U[t,k1]) U[t,k2] (k_spread_lambda's value).  umax[k]: largest finite
-// |re| + |im| of column k.
+// p % nq; value conj(U[t,k1]) U[t,k2] (k_spread_lambda's value).  umax[k]: k_basis_max of U.
 struct LamParts {
   const void* U;
   const float* umax;
@@ -81,7 +87,7 @@ struct LamParts {
     int k2 = 0;
     while ((k2 + 1) * (k2 + 2) / 2 <= p) ++k2;
     const int k1 = p - k2 * (k2 + 1) / 2;
-    return Lane{nt * k1, nt * k2, umax ? fminf(umax[k1] * umax[k2], kFltMax) : 0.f, q};
+    return Lane{nt * k1, nt * k2, umax ? part_bound(umax[k1], umax[k2]) : 0.f, q};
   }
   __device__ __forceinline__ float value(const Lane& L, int, int t) const {
     if (u_complex) {
@@ -96,8 +102,8 @@ struct LamParts {
 
 // Part p of the backprojection: channel p / 2 = (coil c0 + c) K + k, plane p % 2; value
 // y_c conj(U[t,k]) (k_spread_data's value; the tap weights carry the density compensation).
-// tmax[tile][c]: largest component of the tile's samples times their density compensation, infinite
-// if one of them is not finite (bd is NaN then).
+// tmax[tile][c]: largest component of the tile's samples times their density compensation
+// (k_tile_absmax).
 struct DataParts {
   const float2* data;
   const void* U;
@@ -112,9 +118,7 @@ struct DataParts {
   };
   __device__ Lane bind(int part, int tile) const {
     const int ch = part >> 1, c = ch / K, k = ch - c * K;
-    const float tm = tmax ? tmax[(int64_t)tile * nc + c] : 0.f;
-    const float bd = tmax ? fminf(tm * umax[k], kFltMax) : 0.f;
-    return Lane{data + ns_tot * (c0 + c), nt * k, finite_value(tm) ? bd : __int_as_float(0x7fc00000), part & 1};
+    return Lane{data + ns_tot * (c0 + c), nt * k, tmax ? part_bound(tmax[(int64_t)tile * nc + c], umax[k]) : 0.f, part & 1};
   }
   __device__ __forceinline__ float value(const Lane& L, int li, int t) const {
     if (u_complex) {
@@ -126,20 +130,29 @@ struct DataParts {
   }
 };
 
-// umax[k] = max over t of |U[t,k]| (real) or |re| + |im| (complex) where finite; one block per column
-__global__ void k_basis_max(const void* U, int64_t nt, int cplx, float* umax) {
+// used[t] = 1 for the frames (zeroed before) that have a kept sample
+__global__ void k_frames_used(SampleSet S, uint8_t* used) {
+  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < S.n; n += (int64_t)gridDim.x * blockDim.x)
+    used[frame_of(sample_lin(S, n), S.ns_pf)] = 1;
+}
+
+// umax[k] = max over the used frames t (all without `used`) of |U[t,k]| (real) or |re| + |im|
+// (complex), infinite if one of them is not finite; one block per column.  Clears the nbad marks.
+__global__ void k_basis_max(const void* U, int64_t nt, int cplx, const uint8_t* used, float* umax, int* bad, int nbad) {
   __shared__ float red[32];
   const int k = blockIdx.x;
+  for (int i = k * blockDim.x + threadIdx.x; i < nbad; i += gridDim.x * blockDim.x) bad[i] = 0;
   float m = 0.f;
   for (int64_t t = threadIdx.x; t < nt; t += blockDim.x) {
+    if (used && !used[t]) continue;
+    float v;
     if (cplx) {
       const float2 u = reinterpret_cast<const float2*>(U)[t + nt * k];
-      const float v = fabsf(u.x) + fabsf(u.y);
-      if (finite_value(v)) m = fmaxf(m, v);
+      v = fabsf(u.x) + fabsf(u.y);
     } else {
-      const float v = fabsf(reinterpret_cast<const float*>(U)[t + nt * k]);
-      if (finite_value(v)) m = fmaxf(m, v);
+      v = fabsf(reinterpret_cast<const float*>(U)[t + nt * k]);
     }
+    m = finite_value(v) ? fmaxf(m, v) : __int_as_float(0x7f800000);
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
@@ -148,6 +161,21 @@ __global__ void k_basis_max(const void* U, int64_t nt, int cplx, float* umax) {
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, red[w]);
     umax[k] = m;
   }
+}
+
+// umax: K maxima followed by nparts marks
+static int basis_max(const SampleSet& S, const void* U, int cplx, int K, int nparts, DevBuf& umax, cudaStream_t st) {
+  DevBuf used;
+  MRSR_TRY(umax.alloc(sizeof(float) * K + sizeof(int) * nparts));
+  if (S.n < S.ns_pf * S.nt) {  // a mask may have taken all samples of a frame
+    MRSR_TRY(used.alloc(S.nt));
+    MRSR_CHECK_CUDA(cudaMemsetAsync(used.p, 0, S.nt, st));
+    k_frames_used<<<(unsigned)std::min<int64_t>(cdiv(S.n, 256), 152 * 16), 256, 0, st>>>(S, used.as<uint8_t>());
+    MRSR_LAUNCH_CHECK();
+  }
+  k_basis_max<<<K, 256, 0, st>>>(U, S.nt, cplx, used.as<uint8_t>(), umax.as<float>(), umax.as<int>() + K, nparts);
+  MRSR_LAUNCH_CHECK();
+  return MRSR_OK;
 }
 
 // tmax[tile][c] (zeroed before) = largest max(|re|, |im|) * |density compensation| over the
@@ -304,8 +332,10 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
       const typename Parts::Lane L = parts.bind(live ? gpart : 0, item.x);
       // 2^a: bound < 2^ex
       float bd = live ? L.bd : 0.f;
-      bool bad = !(bd >= 0.f);
-      if (bad) bd = 0.f;
+      if (!(bd >= 0.f)) {
+        a.bad[gpart] = 1;
+        bd = 0.f;
+      }
       const int ex = max((int)(__float_as_uint(bd) >> 23), 1) - 126;
       const int ea = min(kSpValBits - ex, 126);
       const float scale = bd > 0.f ? __int_as_float((ea + 127) << 23) : 0.f;
@@ -319,7 +349,6 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
           const float4 en = list[i];
           val[j] = live ? parts.value(L, __float_as_int(en.x), __float_as_int(en.y)) : 0.f;
           if constexpr (D == 3) val[j] *= en.w;
-          bad |= !finite_value(val[j]);
         }
 #pragma unroll
         for (int j = 0; j < 2 * kSpFly; ++j) {
@@ -328,7 +357,6 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
           slots[i * TW + part] = val[j] * scale;
         }
       }
-      if (bad) a.bad[gpart] = 1;
       __syncthreads();
       // The warp's rows, RU apart (a warp near the window's edge, whose rows few samples meet, has
       // another one inside it), meet the samples of ly in [ylo, yhi), one x position at a time:
@@ -430,7 +458,6 @@ static int spread_rows(int d, const int64_t* M, int64_t cells, int nparts, long 
   MRSR_REQUIRE(ts.tile == kSpTile && ts.m0 == (int)M[0] && ts.m1 == (int)M[1] && (d == 2 || ts.m2 == (int)M[2]),
                MRSR_ERR_STATE, "tile sort built for another grid");
   MRSR_REQUIRE(ts.rec.p != nullptr, MRSR_ERR_STATE, "tile sort without tap records");
-  MRSR_CHECK_CUDA(cudaMemsetAsync(bad, 0, sizeof(int) * nparts, st));
   const SpreadRowsArgs a{ts.m0, ts.m1, d == 3 ? ts.m2 : 1, cells, nparts, q, fs, bad, ts.ntx, ts.nty, ts.rec.p,
                          ts.items.as<int4>(), ts.nitems.as<int>(), ts.next.as<unsigned long long>()};
   switch (spread_lanes(nparts)) {
@@ -448,17 +475,14 @@ __global__ void __launch_bounds__(256) k_parts_to_grid(const long long* q, int n
                                                        const FixedScale* fs, const int* bad, float2* out) {
   constexpr int NC = 64;
   __shared__ float tile[P][NC + 1];
-  __shared__ float inv[P];  // 2^-e, NaN for a marked part
+  static_assert(256 % P == 0, "a thread converts one part");
   const int64_t cell0 = (int64_t)blockIdx.x * NC;
   const int grp = blockIdx.y;
   const int nc = cells - cell0 < NC ? (int)(cells - cell0) : NC;
   const long long* qg = q + ((int64_t)grp * cells + cell0) * P;
-  if (threadIdx.x < P) {
-    const int p = grp * P + threadIdx.x;
-    inv[threadIdx.x] = p < nparts && bad[p] ? __int_as_float(0x7fc00000) : fs->inv;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < nc * P; e += 256) tile[e % P][e / P] = fx_to_float(qg[e]) * inv[e % P];
+  const int part = grp * P + threadIdx.x % P;
+  const float inv = part < nparts && bad[part] ? __int_as_float(0x7fc00000) : fs->inv;
+  for (int e = threadIdx.x; e < nc * P; e += 256) tile[e % P][e / P] = fx_to_float(qg[e]) * inv;
   __syncthreads();
   const int ncu = min(P, nparts - grp * P) / nq;  // channels of the group
   for (int e = threadIdx.x; e < ncu * NC; e += 256) {

@@ -44,7 +44,15 @@ def test_basis(mr, cuda, img, K, cplx, value):
     rng, trj, U, data = _scan(img, K, 2, 90, 6, cplx)
     bp = mr.to_host(mr.calculate_backprojection(data, trj, img, U=U))
     lam = mr.to_host(mr.NFFTNormalOp(img, trj, U).Λ)
-    U[np.argmin(np.abs(U[:, 2])), 2] = value
+    t = np.argmin(np.abs(U[:, 2]))
+    U[t, 2] = value
+    # a frame that the mask leaves out
+    mask = np.ones(data.shape[:2], dtype=bool)
+    mask[:, t] = False
+    zero = np.where(np.isfinite(U), U, 0).astype(U.dtype)
+    for call in (lambda u: mr.calculate_backprojection(data, trj, img, U=u, sample_mask=mask),
+                 lambda u: mr.NFFTNormalOp(img, trj, u, sample_mask=mask).Λ):
+        np.testing.assert_array_equal(mr.to_host(call(U)), mr.to_host(call(zero)))
     got = mr.to_host(mr.calculate_backprojection(data, trj, img, U=U))
     assert not np.isfinite(got[:, :, 2]).any()
     keep = [k for k in range(K) if k != 2]
