@@ -6,9 +6,10 @@
 // the R1 inputs x[R2 n1 + n2] in registers, runs an R1-point DFT and applies
 // the twiddle W_L^{n2 f1}.  Step B: one task per (line, f1) holds R2 values
 // and runs an R2-point DFT.  The only shared-memory traffic is the exchange
-// between the two steps.  The R-point DFTs are unrolled Cooley-Tukey
-// compositions of radix 2/3/4/5/8 kernels with twiddles from __constant__
-// tables, so every index is a compile-time constant and stays in registers.
+// between the two steps.  The R-point DFTs are unrolled prime-factor and
+// Cooley-Tukey compositions of radix 2/3/4/5/8 kernels with twiddles from
+// __constant__ tables, so every index is a compile-time constant and stays in
+// registers.
 //
 // Shared-memory slot layout (TC interleaved columns, lo outer lines):
 //   slot(lo, li, a, c) = (lo * R1 + a) * W + c * TC + li,  W = R2*TC + pad
@@ -21,12 +22,13 @@
 namespace mrsr {
 
 // ---------------------------------------------- compile-time factoring ---
+// (20 = 5 * 4: Cartesian 320^2, 12 coils, an apply 66.4 us, as 4 * 5 70.3)
 __host__ __device__ constexpr int rdft_first_factor(int R) {
-  return (R % 8 == 0 && R != 8) ? 8 : (R % 4 == 0 && R != 4) ? 4 : (R % 2 == 0 && R != 2) ? 2
+  return R == 20 ? 5 : (R % 8 == 0 && R != 8) ? 8 : (R % 4 == 0 && R != 4) ? 4 : (R % 2 == 0 && R != 2) ? 2
        : (R % 3 == 0 && R != 3) ? 3 : (R % 5 == 0 && R != 5) ? 5 : R;
 }
 __host__ __device__ constexpr int rdft_table_base(int R) {
-  return (32 % R == 0) ? 32 : (24 % R == 0) ? 24 : (20 % R == 0) ? 20 : (30 % R == 0) ? 30 : (36 % R == 0) ? 36 : (25 % R == 0) ? 25 : 0;
+  return (32 % R == 0) ? 32 : (24 % R == 0) ? 24 : (9 % R == 0) ? 9 : (25 % R == 0) ? 25 : 0;
 }
 
 // exp(S 2 pi i m / R) from the __constant__ tables (S = -1 forward, +1 inverse)
@@ -34,25 +36,44 @@ template <int R, int S>
 __device__ __forceinline__ float2 rtw(int m) {
   constexpr int B = rdft_table_base(R);
   static_assert(B != 0, "no twiddle table for this register DFT length");
-  const float2* t = (B == 32) ? c_tw32 : (B == 24) ? c_tw24 : (B == 20) ? c_tw20 : (B == 30) ? c_tw30 : (B == 36) ? c_tw36 : c_tw25;
+  const float2* t = (B == 32) ? c_tw32 : (B == 24) ? c_tw24 : (B == 9) ? c_tw9 : c_tw25;
   const float2 w = t[(m % R) * (B / R)];
   return make_float2(w.x, S * w.y);
 }
 
+// a^-1 mod m, 0 if a and m share a factor
+__host__ __device__ constexpr int inverse_mod(int a, int m) {
+  for (int i = 1; i < m; ++i)
+    if (a * i % m == 1) return i;
+  return 0;
+}
+
+// R = A B: Cooley-Tukey, or, where A and B have no common factor, the index maps of Good (J. R.
+// Stat. Soc. B 20, 1958) with n = B n1 + A n2 and f = f1 (mod A) = f2 (mod B), which need no
+// twiddles between the two, so no roundings of them either (Cartesian applies, error against
+// float64: 400^2 2.45e-7 -> 2.10e-7, 2.26e-7 with the generic kernels; 200^2 2.32e-7 -> 2.02e-7,
+// 2.12e-7).
 template <int R, int S>
 struct RDft {
   static constexpr int A = rdft_first_factor(R);
   static constexpr int B = R / A;
+  static constexpr bool PF = inverse_mod(A, B) != 0;
+  static constexpr int EA = PF ? B * inverse_mod(B, A) : 1, EB = PF ? A * inverse_mod(A, B) : A;  // f = EA f1 + EB f2
   static __device__ __forceinline__ void run(float2* x) {
     float2 u[R];
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) {
       float2 t[A];
 #pragma unroll
-      for (int n1 = 0; n1 < A; ++n1) t[n1] = x[B * n1 + n2];
+      for (int n1 = 0; n1 < A; ++n1) t[n1] = x[PF ? (B * n1 + A * n2) % R : B * n1 + n2];
       RDft<A, S>::run(t);
 #pragma unroll
-      for (int f1 = 0; f1 < A; ++f1) u[n2 * A + f1] = (n2 * f1 == 0) ? t[f1] : cmul(t[f1], rtw<R, S>(n2 * f1));
+      for (int f1 = 0; f1 < A; ++f1) {
+        if constexpr (PF)
+          u[n2 * A + f1] = t[f1];
+        else
+          u[n2 * A + f1] = (n2 * f1 == 0) ? t[f1] : cmul(t[f1], rtw<R, S>(n2 * f1));
+      }
     }
 #pragma unroll
     for (int f1 = 0; f1 < A; ++f1) {
@@ -61,7 +82,7 @@ struct RDft {
       for (int n2 = 0; n2 < B; ++n2) t[n2] = u[n2 * A + f1];
       RDft<B, S>::run(t);
 #pragma unroll
-      for (int f2 = 0; f2 < B; ++f2) x[f1 + A * f2] = t[f2];
+      for (int f2 = 0; f2 < B; ++f2) x[(EA * f1 + EB * f2) % R] = t[f2];
     }
   }
 };
