@@ -1,4 +1,4 @@
-// Register four-step versions of the apply passes (see fft4.cuh).
+// Register two-step versions of the apply passes (see fft4.cuh).
 //
 // Same data flow as the generic kernels in normalop.cu; each line transform
 // is two register DFT steps with one shared-memory exchange, and the Λ pass

@@ -1,4 +1,4 @@
-// Λ pass of the float32 operator with register four-step transforms (see fft4.cuh):
+// Λ pass of the float32 operator with register two-step transforms (see fft4.cuh):
 // forward FFT along the last axis of K planes of a column tile (the pruned input half
 // zero), the per-voxel K x K kernel product on the spectrum held in the exchange buffer,
 // and the inverse FFT keeping the image half, in place, one (tile, coil) per CTA.

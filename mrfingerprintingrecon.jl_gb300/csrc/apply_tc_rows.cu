@@ -2,7 +2,7 @@
 // on the tensor cores (the Λ pass is in apply_tc.cu; the four-step split and the
 // operand conventions are the same).  One work item is one image row r and one basis
 // index k; the MMA's N vectors are (coil, f1) for every coil of the group.  (The
-// forward row pass stays the float32 four-step kernel, which is faster there.)
+// forward row pass stays the float32 two-step kernel, which is faster there.)
 //
 // Inverse (DFT^-1 along dim 1, crop to 256, conj map, coil sum, alpha / beta):
 //   y[64 m1 + m2] = sum_c conj(S_c) sum_f1 w8^(-m1 f1) w512^(-m2 f1) conj(sum_f2 w64^(m2 f2) conj(Y_c[f1 + 8 f2]))

@@ -6,19 +6,6 @@
 
 namespace mrsr {
 
-// -------------------------------------------------------- dispatch ---
-
-// the first group of lengths (the fp16-storage operator's)
-template <class F>
-inline int with_split(int L, F f) {
-  switch (L) {
-#define MRSR_CASE(L_, R1_, R2_) case L_: return f(Split<R1_, R2_>());
-    MRSR_SPLITS_0(MRSR_CASE)
-#undef MRSR_CASE
-    default: return MRSR_ERR_UNSUPPORTED;
-  }
-}
-
 inline Slots make_slots(int R2, int TC) {
   Slots s;
   s.TC = TC;

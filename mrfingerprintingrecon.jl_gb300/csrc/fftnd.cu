@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(256) k_axis_generic(AxisArgs a) {
   }
 }
 
-// register four-step (compiled lengths)
+// register two-step (compiled lengths)
 template <class SP, int S>
 __global__ void __launch_bounds__(256) k_axis_fast(AxisArgs a, Slots sl) {
   constexpr int R1 = SP::R1, R2 = SP::R2, L = SP::L;

@@ -438,7 +438,7 @@ struct RowTiling {
 };
 
 
-// Rows per CTA of the four-step forward row pass: the smallest count (up to twice the
+// Rows per CTA of the two-step forward row pass: the smallest count (up to twice the
 // line-element budget) whose step-B tasks rpc * lines * R1 best fill the CTA's threads
 // (a multiple of 32, at least 128, at most 256 per round).  For K = 5 lines of 512
 // points this is 2 rows (160 tasks, 160 threads) instead of 1 (80 tasks on 128 threads):
@@ -525,7 +525,7 @@ static int apply_impl(mrsr_normalop* op, const float2* x, float2* y, float2 alph
     const int c0 = grp * op->Cg;
     const int ncg = std::min(op->Cg, g.ncoils - c0);
     // fp16-tc: the inverse row pass runs on the tensor cores too.  The forward row pass stays
-    // the float32 four-step kernel: on 256^2 with 20 coils it takes 0.039 ms against 0.042 ms
+    // the float32 two-step kernel: on 256^2 with 20 coils it takes 0.039 ms against 0.042 ms
     // for a tensor-core form, and adds no fp16 rounding.
     const bool tc_rows = op->precision == MRSR_PREC_FP16_TC && tc_rows_supported(L1, (int)g.n[0], ncg);
     // a stacked operator's planes are independent: without coil maps the rows pass sees

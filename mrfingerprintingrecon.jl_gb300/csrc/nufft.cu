@@ -213,8 +213,8 @@ __device__ __forceinline__ void lane_taps(const SampleSet& S, const int64_t* M, 
   }
 }
 
-// One warp per kept sample (the 3D grids; tile-sorted kernels below do 2D).  A channel's
-// value is formed once per sample; its terms go to the grid as 64-bit atomics.
+// One warp per kept sample, for sets of 2^31 samples or more (the tile-sorted kernels below take the
+// others).  A channel's value is formed once per sample; its terms go to the grid as 64-bit atomics.
 template <int J>
 __global__ void __launch_bounds__(256, 2) k_spread_lambda(SpreadLambdaArgs a, const int* order) {
   const int lane = threadIdx.x & 31;
@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(256, 2) k_spread_lambda(SpreadLambdaArgs a, co
   }
 }
 
+// The same for data channels: also without a basis (each sample then has one channel).
 template <int J>
 __global__ void __launch_bounds__(256, 2) k_spread_data(SpreadDataArgs a, const int* order) {
   const int lane = threadIdx.x & 31;
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(256, 2) k_spread_data(SpreadDataArgs a, const 
   }
 }
 
-// 3D data spreading with a basis into a [cell][part] accumulator (the NP <= 32 parts of a
+// 3D data spreading with a basis, sets of 2^31 samples or more, into a [cell][part] accumulator (the NP <= 32 parts of a
 // coil batch consecutive: re and im of each coil and coefficient).  One warp per sample,
 // lanes over the parts: a lane forms its part's value once, then adds its 512 terms, and
 // the 32 atomics of one warp instruction land on one cell's consecutive parts (a few

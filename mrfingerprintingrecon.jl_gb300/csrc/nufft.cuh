@@ -70,9 +70,10 @@ int es_inv_psi_table(int64_t M, int64_t jmin, int64_t count, const float** out);
 
 // Fixed-point accumulation of the spread grids.  Each tap's term (a float32 product of
 // the sample value and the kernel weights) is scaled by 2^e, rounded to an integer and
-// added to a 64-bit grid with integer atomics.  Integer addition is associative, so every
-// cell holds the exact sum of its rounded terms whatever order the samples land in: the
-// grids are bitwise reproducible run to run, and the sum carries no accumulation error (a
+// added to a 64-bit grid with integer atomics.  (The register rows of spread_rows.cuh round
+// values and taps instead, sum a chunk's products exactly and round each chunk's sum once.)
+// Integer addition is associative, so a cell holds the same sum whatever order the samples
+// land in: the grids are bitwise reproducible run to run, and the sum carries no accumulation error (a
 // float32 atomic sum of n terms drifts by ~sqrt(n) float32 roundings of the running total,
 // a float64 one by ~n float64 roundings).  e = min(62 - ceil(log2(n_terms max|term|)),
 // 40 - ceil(log2(max|term|))) from a device-side bound: no cell sum can leave 63 bits, no

@@ -1,5 +1,5 @@
 // Kernel arguments of the apply passes and the per-voxel K x K product,
-// shared by the generic (Stockham) and the register four-step kernels.
+// shared by the generic (Stockham) and the register two-step kernels.
 #pragma once
 #include "normalop.cuh"
 
@@ -32,7 +32,7 @@ struct LamPassArgs {
   const void* lam;     // [tile][chunk][P][FC][TC]
   float2* stack;       // planes [cl][k][row][inner], in place
   int FC, NCH;         // Λ chunk: frequencies per chunk, chunks per tile (L = FC * NCH)
-  int ncg = 1;         // coils of the launch (four-step kernel: block = tile * ncg + coil)
+  int ncg = 1;         // coils of the launch (two-step kernel: block = tile * ncg + coil)
   FastDiv fcd;         // division by FC
 };
 

@@ -47,7 +47,6 @@ constexpr int kWinCells = kSpWin * kSpWin;
 constexpr int kSpWarps = 12;
 constexpr int kSpThreads = kSpWarps * 32;
 constexpr int kSpChunk = kSpThreads;          // samples of a chunk, at most: one per thread
-constexpr int kSpFly = 1;                     // samples a warp stages at once
 constexpr int kSpValBits = 29, kSpTapBits = 25;
 static_assert((unsigned long long)kSpChunk << (kSpValBits + kSpTapBits) < 7ull << 60, "a chunk's sums must fit in 63 bits");
 
@@ -297,33 +296,19 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
     if (key >= 0) list[start[key] + rank] = ent;
     __syncthreads();
     // taps of the staged samples, a warp each
-    for (int i0 = warp; i0 < ns; i0 += kSpWarps * kSpFly) {
-      float tap[kSpFly];
-      int pl[kSpFly];
-#pragma unroll
-      for (int j = 0; j < kSpFly; ++j) {
-        const int i = i0 + j * kSpWarps;
-        if (i >= ns) break;
-        pl[j] = __float_as_int(list[i].z);                 // ly | lx << 4 | place in the item << 8
-        const int dy = lane - kEsWidth - (pl[j] & 15);     // lanes 8 .. 31: rows 0 .. 23
-        const Rec& r = recs[item.y + (pl[j] >> 8)];
-        tap[j] = 0.f;
-        if (lane < kEsWidth)
-          tap[j] = r.wx[lane];
-        else if ((unsigned)dy < (unsigned)kEsWidth)
-          tap[j] = r.wy[dy];
-      }
-#pragma unroll
-      for (int j = 0; j < kSpFly; ++j) {
-        const int i = i0 + j * kSpWarps;
-        if (i >= ns) break;
-        if (lane < kEsWidth) {
-          const int w = __float2int_rn(tap[j] * (float)(1 << kSpTapBits));
-          reinterpret_cast<int*>(slots)[i * TW + TX + lane] = w;
-          atomicAdd(&csum[(pl[j] & 15) * (kSpWin + 1) + ((pl[j] >> 4) & 15) + lane], (unsigned long long)w);
-        } else {
-          slots[i * TW + TX + lane] = tap[j];
-        }
+#pragma unroll 1
+    for (int i = warp; i < ns; i += kSpWarps) {
+      const int pl = __float_as_int(list[i].z);         // ly | lx << 4 | place in the item << 8
+      const int dy = lane - kEsWidth - (pl & 15);       // lanes 8 .. 31: rows 0 .. 23
+      const Rec& r = recs[item.y + (pl >> 8)];
+      const float* src = lane < kEsWidth ? r.wx + lane : r.wy + dy;  // one load for all lanes
+      const float tap = lane < kEsWidth || (unsigned)dy < (unsigned)kEsWidth ? *src : 0.f;
+      if (lane < kEsWidth) {
+        const int w = __float2int_rn(tap * (float)(1 << kSpTapBits));
+        reinterpret_cast<int*>(slots)[i * TW + TX + lane] = w;
+        atomicAdd(&csum[(pl & 15) * (kSpWin + 1) + ((pl >> 4) & 15) + lane], (unsigned long long)w);
+      } else {
+        slots[i * TW + TX + lane] = tap;
       }
     }
     for (int grp = 0; grp < ngroups; ++grp) {
@@ -339,11 +324,11 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
       const int ex = max((int)(__float_as_uint(bd) >> 23), 1) - 126;
       const int ea = min(kSpValBits - ex, 126);
       const float scale = bd > 0.f ? __int_as_float((ea + 127) << 23) : 0.f;
-      // values of the staged samples
-      for (int i0 = warp * RW + rsub; i0 < ns; i0 += RU * 2 * kSpFly) {
-        float val[2 * kSpFly];
+      // values of the staged samples, two at a time
+      for (int i0 = warp * RW + rsub; i0 < ns; i0 += RU * 2) {
+        float val[2];
 #pragma unroll
-        for (int j = 0; j < 2 * kSpFly; ++j) {
+        for (int j = 0; j < 2; ++j) {
           const int i = i0 + j * RU;
           if (i >= ns) break;
           const float4 en = list[i];
@@ -351,7 +336,7 @@ __global__ void __launch_bounds__(kSpThreads, 2) k_spread_rows(SpreadRowsArgs a,
           if constexpr (D == 3) val[j] *= en.w;
         }
 #pragma unroll
-        for (int j = 0; j < 2 * kSpFly; ++j) {
+        for (int j = 0; j < 2; ++j) {
           const int i = i0 + j * RU;
           if (i >= ns) break;
           slots[i * TW + part] = val[j] * scale;
