@@ -95,8 +95,8 @@ struct DevBuf {
 // 203, 384^2, 32 coils 1524 -> 1458 (with a two-step Λ pass).  Not where a grid has less than two
 // blocks an SM (64^2, 4 coils: the host's launches bound it, and this kind takes longer) nor
 // where it runs tens of waves, of which only the first gains and every block pays for the wait
-// (128^3: 10.65 -> 11.22 ms), nor in captured graphs (CG 1.73 -> 1.78 ms), nor for the three-step kernels, whose first statement
-// is the load that has to wait (256^2, 20 coils 207.5 -> 208.4 us).
+// (128^3: 10.65 -> 11.22 ms), nor in captured graphs (CG 1.73 -> 1.78 ms), nor for the three-step
+// kernels, whose first statement is the load that has to wait (256^2, 20 coils 207.5 -> 208.4 us).
 constexpr unsigned kPdlMinBlocks = 304, kPdlMaxBlocks = 4096;
 __device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
