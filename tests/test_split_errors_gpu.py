@@ -29,3 +29,19 @@ def _error(mr, n, seed, K=2, nc=3):
 @pytest.mark.parametrize("n", sorted(GENERIC))
 def test_error(mr, cuda, n):
     assert 0.5 * (_error(mr, n, 0) + _error(mr, n, 1)) <= 1.03e-7 * GENERIC[n]
+
+
+# the same for zero-padded operators on n x n images (2 n points a line), 3 coefficients, 8 coils
+GENERIC_PADDED = {36: 0.844, 60: 0.694, 72: 0.838, 100: 0.739, 180: 0.788, 200: 0.738, 250: 1.058, 288: 1.032}
+
+
+@pytest.mark.parametrize("n", sorted(GENERIC_PADDED))
+def test_padded_error(mr, cuda, n):
+    cases = pytest.importorskip("perf.cases")
+    case = dict(kind="apply", n1=n, n2=n, n3=0, K=3, coils=8, basis="real", nt=0, spokes=1, iters=0)
+    total = 0.0
+    for seed in (1, 2):
+        y, ref = cases.run(cases.prepare(case, seed)), cases.exact(case, seed)
+        y, ref = (t[0] if isinstance(t, (list, tuple)) else t for t in (y, ref))
+        total += float((y.to(ref.dtype).reshape(ref.shape) - ref).norm() / ref.norm())
+    assert 0.5 * total <= 1.03e-7 * GENERIC_PADDED[n]
